@@ -671,6 +671,7 @@ int gpv_context_reserve(gpv_context *ctx, int64_t n_subsets, int32_t max_radius,
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     if (int rc = ensure_tables(ctx, max_radius)) return rc;
+    if (int rc = ensure_run_tables(ctx, max_radius)) return rc;  // no allocation left for a solve that a caller captures
     const int64_t npx = ctx->h_tab_n[max_radius];
     const int64_t stride = 4 * ((npx + 31) / 32 * 32);
     // enough for either kernel: 8 B per element, one slot per resident warp

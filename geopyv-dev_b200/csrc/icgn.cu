@@ -22,7 +22,10 @@
 //    B_j = sum SDI_ij g~_i.
 //  * icgn_fp64   -- the plain form: one thread block per subset, FP64
 //    throughout on FP64 coefficients, and the reference's three sweeps per
-//    iteration (g_m, then delta_g, then the fused update + ZNSSD).
+//    iteration (g_m, then delta_g, then the fused update + ZNSSD); runs the
+//    FP64 solves that ask for the rigid-texture template.  fagn_kernel below
+//    is the same for FAGN.  The deformable template takes the run layout
+//    (icgn_runs64.cu).
 #include <cstdlib>
 
 #include "icgn_common.cuh"
@@ -851,7 +854,7 @@ int eval_launch(const gpv_image *img, const double *xy_dev, int64_t n, int preci
     return GPV_SUCCESS;
 }
 
-int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s);
+int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cudaStream_t s);
 
 // GPV_MIXED_KERNEL=warp selects the warp-per-subset kernel for the mixed
 // precision solve (default: block per subset with a staged window).
@@ -903,6 +906,10 @@ int solve_launch(gpv_context *ctx, const SolveLaunch &L, cudaStream_t s) {
             A.f64 = nullptr;
             A.g64 = nullptr;
         }
+        if (!(prm->flags & GPV_SOLVE_RIGID_TEXTURE)) {
+            if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (96 + (size_t)L.n))) return rc;
+            return tile_launch(ctx, A, L.n, SolveForm::kFagn, s);
+        }
         int per_sm = 0;
         GPV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fagn_kernel, kFp64Threads, 0));
         if (per_sm < 1) per_sm = 1;
@@ -918,9 +925,10 @@ int solve_launch(gpv_context *ctx, const SolveLaunch &L, cudaStream_t s) {
         GPV_CUDA_TRY(cudaGetLastError());
         return GPV_SUCCESS;
     }
-    if (!fp64 && !use_warp_kernel()) {
+    const bool runs64 = fp64 && !(prm->flags & GPV_SOLVE_RIGID_TEXTURE);
+    if (runs64 || (!fp64 && !use_warp_kernel())) {
         if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (96 + (size_t)L.n))) return rc;
-        return tile_launch(ctx, A, L.n, s);
+        return tile_launch(ctx, A, L.n, runs64 ? SolveForm::kFp64 : SolveForm::kMixed, s);
     }
     int workers, threads;
     size_t elem;

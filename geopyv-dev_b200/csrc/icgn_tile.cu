@@ -1292,7 +1292,11 @@ int query_nsmid(int *out) {
 // Launch one kernel per (order, radius class) segment that can hold
 // subsets, spread over the context stream and its two auxiliary streams;
 // kernels sharing a stream run one after the other and share its scratch.
-int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s) {
+// form: the mixed-precision solve, or one of the FP64 run-layout solves
+// (persistent grids, deformable template; FAGN on FP64 coefficients when K
+// has them).
+int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cudaStream_t s) {
+    const bool mixed = form == SolveForm::kMixed, fagn = form == SolveForm::kFagn;
     int32_t *ws = static_cast<int32_t *>(ctx->tile_ws.ptr);
     int32_t *cnt = ws, *fill = ws + 16, *seg = ws + 32, *queues = ws + 64, *order_out = ws + 96;
     GPV_CUDA_TRY(cudaMemsetAsync(ws, 0, 96 * sizeof(int32_t), s));
@@ -1306,23 +1310,44 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s) {
         bool runs = false;               // the run-layout kernel (icgn_runs.cu), run length run_k
         int run_k = 0, nslot = 0;
         int64_t stride = 0;
+        size_t smem = 0;                 // window bytes
+        const void *fn = nullptr;
         bool live = false;
     };
     Plan plan[kSegs];
     int64_t region = 0;  // scratch floats per stream: its largest launch
     // one block per subset when the context asks for it and the host knows
     // the segment sizes (host batches); else a persistent grid
-    const bool per_subset = (ctx->flags & GPV_CONTEXT_PER_SUBSET_BLOCKS) && ctx->seg_count_valid && ctx->n_smid > 0;
+    const bool per_subset = mixed && (ctx->flags & GPV_CONTEXT_PER_SUBSET_BLOCKS) && ctx->seg_count_valid && ctx->n_smid > 0;
     for (int q = 0; q < kSegs; q++) {
         const int order = 2 - q / kRClasses, c = q % kRClasses;
         const int lo = c == 0 ? 0 : kRBoundHost[c - 1];
         Plan &P = plan[q];
         // the rigid template runs on persistent grids (orders 1 and 2)
-        P.rigid = (K.flags & GPV_SOLVE_RIGID_TEXTURE) && order >= 1;
+        P.rigid = mixed && (K.flags & GPV_SOLVE_RIGID_TEXTURE) && order >= 1;
         P.ps = per_subset && !P.rigid;
         P.live = lo < K.max_radius && ((ctx->seg_mask >> q) & 1u) && (!P.ps || ctx->seg_count[q] > 0);
         if (!P.live) continue;
         P.rmax = std::min(kRBoundHost[c], K.max_radius);
+        if (!mixed) {
+            // FP64 run layout: 3 blocks of 128 threads per SM up to radius 32 (the
+            // windows of three blocks fit), 256 threads where fewer windows fit
+            P.nt = P.rmax > 32 ? 256 : 128;
+            P.run_k = run64_run_length();
+            if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
+            P.fn = run64_kernel(order, P.nt, fagn, K.f64 != nullptr);
+            int max_bytes = 0;
+            if (int rc = allow_max_dynamic_smem(P.fn, &max_bytes)) return rc;
+            P.cap = std::min(run64_window_cap(P.rmax), max_bytes / (int)sizeof(double) / 4 * 4);
+            P.smem = sizeof(double) * (size_t)P.cap;
+            GPV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P.per_sm, P.fn, P.nt, P.smem));
+            if (P.per_sm < 1) { set_error("subset window does not fit in shared memory"); return GPV_ERR_INVALID; }
+            run_scratch_floats(ctx, P.rmax, P.run_k, &P.nslot);
+            P.stride = 2 * run64_scratch_doubles(P.nslot, fagn);  // floats
+            P.blocks = (int)std::min<int64_t>((int64_t)P.per_sm * ctx->num_sms, n);
+            region = std::max(region, P.blocks * P.stride);
+            continue;
+        }
         P.nt = tile_threads_for(ctx, P.rmax);
         P.layout = tile_layout_for(ctx, P.rmax);
         // persistent deformable segments run the run-layout kernel unless
@@ -1377,7 +1402,9 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s) {
         }
         region = std::max(region, slots * P.stride);
     }
-    if (int rc = ctx->scratch.ensure((size_t)3 * region * sizeof(float))) return rc;
+    // FP64 records of large radii: one stream's scratch when three would pass 4 GB
+    const int nstream = !mixed && 3 * region * (int64_t)sizeof(float) > (int64_t(4) << 30) ? 1 : 3;
+    if (int rc = ctx->scratch.ensure((size_t)nstream * region * sizeof(float))) return rc;
     GPV_CUDA_TRY(cudaEventRecord(ctx->ev[0], s));
     cudaStream_t st[3] = {s, ctx->aux[0], ctx->aux[1]};
     bool used[3] = {true, false, false};
@@ -1390,7 +1417,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s) {
         // no long tail and stay on the caller's stream (fewer streams share
         // the device's hardware queues with other contexts' work)
         const int k = P.ps ? 0 : next;
-        next = (next + 1) % 3;
+        next = (next + 1) % nstream;
         if (!used[k]) {
             GPV_CUDA_TRY(cudaStreamWaitEvent(st[k], ctx->ev[0], 0));
             used[k] = true;
@@ -1409,7 +1436,10 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, cudaStream_t s) {
         T.slots_per_sm = P.per_sm;
         T.n_mask = ctx->n_smid;
         const size_t smem = sizeof(float) * P.cap;
-        if (P.runs) {
+        if (!mixed) {
+            T.k.scratch_stride = P.stride / 2;  // doubles
+            if (int rc = run64_launch(ctx, P.fn, P.nt, P.blocks, P.smem, st[k], T.k, T.seg, T.queue, P.cap, P.nslot)) return rc;
+        } else if (P.runs) {
             if (int rc = run_launch(ctx, 2 - q / kRClasses, P.nt, P.run_k, (K.flags & GPV_SOLVE_KAHAN) != 0, P.blocks,
                                     smem, st[k], T.k, T.seg, T.queue, P.cap, P.nslot, T.slot_mask, T.slots_per_sm,
                                     T.n_mask))

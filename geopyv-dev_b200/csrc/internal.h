@@ -177,6 +177,7 @@ struct SolveLaunch {
     int max_radius;
 };
 int solve_launch(gpv_context *ctx, const SolveLaunch &L, cudaStream_t s);
+enum class SolveForm { kMixed, kFp64, kFagn };
 int eval_launch(const gpv_image *img, const double *xy_dev, int64_t n, int precision, double *out_dev,
                 cudaStream_t s);
 int ensure_tables(gpv_context *ctx, int max_radius);
@@ -204,12 +205,20 @@ int query_nsmid(int *out);
 // time, runs of K template pixels per lane)
 int ensure_run_tables(gpv_context *ctx, int max_radius);
 int run_window_cap(int rmax, int K);
+int run_length_index(int K);
 int64_t run_scratch_floats(gpv_context *ctx, int rmax, int K, int *nslot);
 const void *run_kernel(int order, int nt, int K, bool per_subset, bool kahan);
 struct KArgs;
 int run_launch(gpv_context *ctx, int order, int nt, int K, bool kahan, int blocks, size_t smem, cudaStream_t s,
                const KArgs &k, const int32_t *seg, int *queue, int win_cap, int nslot, uint32_t *slot_mask,
                int slots_per_sm, int n_mask);
+// icgn_runs64.cu: the FP64 solves (ICGN, FAGN) in run layout
+int run64_run_length();
+int run64_window_cap(int rmax);
+int64_t run64_scratch_doubles(int nslot, bool fagn);
+const void *run64_kernel(int order, int nt, bool fagn, bool c64);
+int run64_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,
+                 const int32_t *seg, int *queue, int win_cap, int nslot);
 // Run length of the run-layout kernel for subsets up to max_radius
 // (GPV_RUN_K, else a candidate being timed, else the tuned choice, else 4).
 int run_length_for(gpv_context *ctx, int max_radius);
