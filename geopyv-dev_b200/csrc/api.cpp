@@ -289,7 +289,7 @@ static void context_release(gpv_context *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (DevBuf *b : {&ctx->offs, &ctx->slots, &ctx->tab_off, &ctx->tab_n, &ctx->scratch, &ctx->queue, &ctx->desc_dev, &ctx->out_dev,
                       &ctx->order_dev, &ctx->hist_dev, &ctx->eval_dev, &ctx->tile_ws, &ctx->slot_mask,
-                      &ctx->run_tasks, &ctx->run_off, &ctx->run_n})
+                      &ctx->run_tab})
         b->release();
     ctx->h_stage.release();
     for (int k = 0; k < 2; k++)
@@ -849,15 +849,16 @@ int gpv_solve_batch_device(gpv_context *ctx, const gpv_image *f, const gpv_image
 
 }  // extern "C"
 
-// Addresses of the context workspace a captured solve reads and writes.
+// Addresses of the context workspace a captured solve reads and writes, and
+// the radius its run tables reach (their layout depends on it).
 struct WorkspaceAddrs {
-    const void *p[11];
+    const void *p[10];
     bool operator==(const WorkspaceAddrs &o) const { return std::memcmp(p, o.p, sizeof p) == 0; }
 };
 static WorkspaceAddrs workspace_addrs(const gpv_context *ctx) {
     return WorkspaceAddrs{{ctx->scratch.ptr, ctx->queue.ptr, ctx->tile_ws.ptr, ctx->offs.ptr, ctx->slots.ptr,
-                           ctx->tab_off.ptr, ctx->tab_n.ptr, ctx->slot_mask.ptr, ctx->run_tasks.ptr, ctx->run_off.ptr,
-                           ctx->run_n.ptr}};
+                           ctx->tab_off.ptr, ctx->tab_n.ptr, ctx->slot_mask.ptr, ctx->run_tab.ptr,
+                           reinterpret_cast<const void *>((uintptr_t)ctx->run_table_radius)}};
 }
 
 struct gpv_batch_graph {
@@ -1055,14 +1056,13 @@ int gpv_autotune(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const
     p.precision = GPV_PREC_MIXED;
     p.history = nullptr;
     p.flags &= ~(GPV_SOLVE_ETA | GPV_SOLVE_FAGN | GPV_SOLVE_RIGID_TEXTURE);  // the tuned kernel is the mixed ICGN one
-    // candidates: threads per block x run length (run-layout kernel), or
-    // threads per block x template layout (compact, 8 x 4 tiles) when the
-    // tiled kernel is selected
+    // candidates: threads per block (run-layout kernel), or threads per block x
+    // template layout (compact, 8 x 4 tiles) when the tiled kernel is selected
     const bool runs = use_run_kernel();
-    static const int cand_runs[6][2] = {{128, 8}, {256, 8}, {128, 4}, {256, 4}, {64, 4}, {64, 8}};
+    static const int cand_runs[3][2] = {{128, 4}, {256, 4}, {64, 4}};
     static const int cand_tile[4][2] = {{128, 0}, {256, 0}, {128, 2}, {256, 2}};
     const int(*cand)[2] = runs ? cand_runs : cand_tile;
-    const int ncand = runs ? 6 : 4;
+    const int ncand = runs ? 3 : 4;
     for (int c = 0; c < 3; c++) {
         if (threads_out) threads_out[c] = 0;
         if (cls[c].empty()) continue;
@@ -1078,7 +1078,6 @@ int gpv_autotune(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const
             const int t = cd[0];
             ctx->force_threads = t;
             ctx->force_layout = runs ? -1 : cd[1];
-            ctx->force_run_k = runs ? cd[1] : 0;
             double ms_best = 1e300;
             for (int rep = 0; rep < 3; rep++) {
                 cudaEvent_t e0, e1;
@@ -1092,7 +1091,7 @@ int gpv_autotune(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const
                 cudaEventElapsedTime(&ms, e0, e1);
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
-                if (rc) { ctx->force_threads = 0; ctx->force_layout = -1; ctx->force_run_k = 0; return rc; }
+                if (rc) { ctx->force_threads = 0; ctx->force_layout = -1; return rc; }
                 if (rep > 0) ms_best = std::min(ms_best, (double)ms);
             }
             if (ms_best < best) {
@@ -1104,7 +1103,6 @@ int gpv_autotune(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const
         }
         ctx->force_threads = 0;
         ctx->force_layout = -1;
-        ctx->force_run_k = 0;
         ctx->tuned_threads[c] = best_nt;
         ctx->tuned_layout[c] = best_layout;
         ctx->tuned_run_k[c] = best_k;

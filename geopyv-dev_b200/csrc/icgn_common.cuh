@@ -196,51 +196,57 @@ __device__ __noinline__ bool compose2(const double *p, const double *d, double *
 }
 
 // Order-2 composition in registers, fully unrolled: solve W_delta^T X = R^T
-// by Gaussian elimination without pivoting.  The lifted warp of a
-// translation is unit upper triangular, and with strain / curvature terms of
-// an increment it stays close to that, so the pivots stay near 1; a zero or
-// non-finite pivot reports W_delta singular.
+// by Gaussian elimination without pivoting.  W_delta's last row is (0, .., 0, 1),
+// so the first five unknowns form a system of their own and the sixth follows.
+// The lifted warp of a translation is unit upper triangular, and with strain /
+// curvature terms of an increment it stays close to that, so the pivots stay
+// near 1; a zero or non-finite pivot reports W_delta singular.
 __device__ __forceinline__ bool compose2_regs(const double *p, const double *d, double *out) {
     double W[36];
     lifted(d, W);
-    double A[6][6], X[6][2];
+    double A[5][5], X[5][2];
 #pragma unroll
-    for (int i = 0; i < 6; i++)
+    for (int i = 0; i < 5; i++)
 #pragma unroll
-        for (int j = 0; j < 6; j++) A[i][j] = W[j * 6 + i];
+        for (int j = 0; j < 5; j++) A[i][j] = W[j * 6 + i];
     X[0][0] = 0.5 * p[6]; X[0][1] = 0.5 * p[7];
     X[1][0] = p[8];       X[1][1] = p[9];
     X[2][0] = 0.5 * p[10]; X[2][1] = 0.5 * p[11];
     X[3][0] = 1.0 + p[2]; X[3][1] = p[3];
     X[4][0] = p[4];       X[4][1] = 1.0 + p[5];
-    X[5][0] = p[0];       X[5][1] = p[1];
     bool ok = true;
+    double inv[5];
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
+    for (int k = 0; k < 5; k++) {
         const double piv = A[k][k];
         ok = ok && (piv != 0.0) && isfinite(piv);
-        const double inv = __drcp_rn(piv);  // the correctly rounded 1 / piv, without a general division
+        inv[k] = __drcp_rn(piv);  // the correctly rounded 1 / piv, without a general division
 #pragma unroll
-        for (int i = k + 1; i < 6; i++) {
-            const double f = A[i][k] * inv;
+        for (int i = k + 1; i < 5; i++) {
+            const double f = A[i][k] * inv[k];
 #pragma unroll
-            for (int j = k + 1; j < 6; j++) A[i][j] = fma(-f, A[k][j], A[i][j]);
+            for (int j = k + 1; j < 5; j++) A[i][j] = fma(-f, A[k][j], A[i][j]);
             X[i][0] = fma(-f, X[k][0], X[i][0]);
             X[i][1] = fma(-f, X[k][1], X[i][1]);
         }
     }
 #pragma unroll
-    for (int k = 5; k >= 0; k--) {
+    for (int k = 4; k >= 0; k--) {
 #pragma unroll
-        for (int j = k + 1; j < 6; j++) {
+        for (int j = k + 1; j < 5; j++) {
             X[k][0] = fma(-A[k][j], X[j][0], X[k][0]);
             X[k][1] = fma(-A[k][j], X[j][1], X[k][1]);
         }
-        const double inv = __drcp_rn(A[k][k]);
-        X[k][0] *= inv;
-        X[k][1] *= inv;
+        X[k][0] *= inv[k];
+        X[k][1] *= inv[k];
     }
-    out[0] = X[5][0]; out[1] = X[5][1];
+    double u = p[0], v = p[1];
+#pragma unroll
+    for (int j = 0; j < 5; j++) {
+        u = fma(-W[j * 6 + 5], X[j][0], u);
+        v = fma(-W[j * 6 + 5], X[j][1], v);
+    }
+    out[0] = u; out[1] = v;
     out[2] = X[3][0] - 1.0; out[3] = X[3][1];
     out[4] = X[4][0]; out[5] = X[4][1] - 1.0;
     out[6] = 2.0 * X[0][0]; out[7] = 2.0 * X[0][1];

@@ -32,6 +32,19 @@
 //    matrix, FP64, one warp), and its inverse formed from the factor
 //    (H^-1 = D L^-T L^-1 D); each iteration's increment is that inverse times
 //    the gradient (FP64, 12 lanes).
+//  * Instruction fetch.  An SM caches 32 KB of instructions (8 KB next to each
+//    scheduler); past that they come from a cache that several SMs share, and
+//    that cache was 81 % busy: the solve's blocks walk some 100 KB of code, each
+//    in its own phase.  So the stretches run once or a few times per subset
+//    are kept short -- the factor as passes of rolled loops, the sums over lanes
+//    through shared memory instead of unrolled shuffles, the omitted-mode
+//    diagnostic only in the kernels of launches that ask for it.  Measured with
+//    the loads of records past L1 (they are read once per iteration) and the
+//    floors by rounding: 37-40k second-order subsets of radius 30 / 24 / 16
+//    5.71 -> 5.36, 4.80 -> 4.23, 3.99 -> 3.24 ms, 27k first-order ones of
+//    radius 25 2.35 -> 2.18 ms; the shared cache 67 % busy.  A pool of 16 warps per
+//    SM sharing five subsets (no block barriers) measured 2.6 times slower: its
+//    warps fetch each stretch alone, at 93 % of that cache.
 //  * Sums.  The per-iteration sums (g - f_m, its square, (f - f_m)(g - f_m)
 //    and the steepest-descent products) are FP32 over one run (at most K
 //    samples), then FP64 per thread and across the block in a fixed order
@@ -51,15 +64,15 @@
 namespace gpv {
 namespace {
 
-constexpr int kRunMaxWarps = 8;  // blocks of 64, 128 or 256 threads
-constexpr int kRunLengths[2] = {4, 8};  // run lengths K with task tables
+constexpr int kBufPitch = 9;  // a warp's staging of sums over lanes: 32 rows of 8 values
 
 // NW: warps per block (block sums are kept per warp)
 template <int NW>
 struct RunSmem {
     double mom[3 * 15];
-    double L[144];     // Cholesky factor of the scaled Hessian, then its inverse (row-major)
-    double Hi[144];    // the Hessian, replaced by H^-1 formed from the factor
+    double L[144];     // the Cholesky factor's inverse (row-major)
+    double Hi[160];    // the factor's columns, then H^-1
+    float part[NW][32 * kBufPitch];  // per-warp staging of the sums over lanes
     double linv[12];   // 1 / L_jj
     double dsc[12];    // Jacobi scale 1 / sqrt(H_jj)
     double A[12], S[12];
@@ -75,72 +88,102 @@ struct RunSmem {
     int win_r0, win_c0, win_h, win_w, win_p, win_ok;
 };
 
-
-// Copy coefficient rows [r0, r0+wh) x cols [c0, c0+ww) (c0, ww multiples of
-// 4) into win with row pitch `pitch`; out-of-range rows / columns clamped.
-// Threads [t0, NT) issue asynchronous 16-byte global-to-shared copies
+// Plan g's or f's window over pixels [xlo, xhi] x [ylo, yhi] and stage it in
+// win by threads [t0, NT): 16-byte asynchronous global-to-shared copies
 // (cp.async, no registers held for the data), so all of a thread's copies
-// are in flight at once; each thread waits for its own copies before it
-// returns, and the caller's block barrier publishes the window.  Both
-// addresses are 16-byte aligned: coefficient rows are a multiple of 32 floats
-// apart, c0 and the clamped columns are multiples of 4, and the window's
-// pitch is a multiple of 4 floats (run_pitch).
+// are in flight at once; rows and columns outside the coefficients are
+// clamped.  Each thread waits for its own copies before it returns, and the
+// caller's block barrier publishes the window and its place in sm (win_ok:
+// it fits and is staged).  Both addresses are 16-byte aligned: coefficient rows
+// are a multiple of 32 floats apart, c0 and the clamped columns are multiples
+// of 4, and the window's pitch is a multiple of 4 floats (run_pitch).
 template <int NT>
-__device__ __forceinline__ void run_stage(const float *__restrict__ C, int64_t cpitch, int ch, int r0, int c0, int wh,
-                                          int ww, int pitch, float *win, int t0) {
-    const int nv = ww >> 2;
-    for (int idx = (int)threadIdx.x - t0; idx < wh * nv; idx += NT - t0) {
-        const int rr = idx / nv, cc = (idx - rr * nv) << 2;
-        int row = r0 + rr;
-        row = row < 0 ? 0 : (row > ch - 1 ? ch - 1 : row);
-        int col = c0 + cc;
-        col = col < 0 ? 0 : (col > (int)cpitch - 4 ? (int)cpitch - 4 : col);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(win + rr * pitch + cc);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(C + (int64_t)row * cpitch + col)
-                     : "memory");
+__device__ __forceinline__ void place_window(RunSmem<NT / 32> &sm, const float *__restrict__ C, int64_t cpitch, int ch,
+                                             int border, int cap, int xlo, int xhi, int ylo, int yhi, float *win, int t0) {
+    int r0, c0, wh, ww, pitch;
+    const bool ok = run_plan<32>(xlo, xhi, ylo, yhi, border, cap, r0, c0, wh, ww, pitch);
+    if (ok) {
+        const int nv = ww >> 2;
+#pragma unroll 2
+        for (int idx = (int)threadIdx.x - t0; idx < wh * nv; idx += NT - t0) {
+            const int rr = idx / nv, cc = (idx - rr * nv) << 2;
+            const int row = max(min(r0 + rr, ch - 1), 0), col = max(min(c0 + cc, (int)cpitch - 4), 0);
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(win + rr * pitch + cc);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(C + (int64_t)row * cpitch + col)
+                         : "memory");
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if ((int)threadIdx.x == t0) {
+        sm.win_ok = ok;
+        sm.win_r0 = r0; sm.win_c0 = c0; sm.win_h = wh; sm.win_w = ww; sm.win_p = pitch;
+    }
 }
 
-// Warp sums of K FP32 per-thread values (FP64 totals) into dst[0..K).
-template <int KV, int C = 0>
-__device__ __forceinline__ void run_warp_sums(const float (&a)[KV], double *dst, int lane) {
-    if constexpr (C < KV) {
-        constexpr int N = (KV - C) < 16 ? (KV - C) : 16;
-        double v[N];
+// Sums over a warp's lanes (FP64) of up to 8 columns of its staging buffer
+// (32 rows, pitch 9: no bank conflicts either way) into dst[0 .. g): eight
+// lanes per quarter of the rows, two chains a lane.
+__device__ __forceinline__ void column_sums(const float *buf, double *dst, int g, int lane) {
+    const float *p = buf + (lane >> 3) * (8 * kBufPitch) + (lane & 7);
+    double s0 = (double)p[0], s1 = (double)p[kBufPitch];
 #pragma unroll
-        for (int j = 0; j < N; j++) v[j] = (double)a[C + j];
-        warp_sum_many<N>(v, dst + C, lane);
-        run_warp_sums<KV, C + N>(a, dst, lane);
+    for (int i = 2; i < 8; i += 2) {
+        s0 += (double)p[i * kBufPitch];
+        s1 += (double)p[(i + 1) * kBufPitch];
     }
+    s0 += s1;
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 8);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
+    if (lane < g) dst[lane] = s0;
 }
 
-template <int NT>
-__device__ __forceinline__ double run_block_sum(double v, RunSmem<NT / 32> &sm) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const double s = warp_sum(v);
-    if (lane == 0) sm.red[wid][0] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
+// Warp sums (FP64) of N FP32 values per lane into dst[0..N) through the
+// warp's staging buffer, 8 at a time.  A butterfly of shuffles per 16 values
+// took 2.4 times the instructions (64-bit shuffles are two each).  ROLLED: the
+// values pass through local memory so that the groups are passes of one
+// loop: the setup's 73 values would otherwise unroll to ten copies.
+template <int N, bool ROLLED>
+__device__ __forceinline__ void run_warp_sums(const float (&a)[N], float *buf, double *dst, int lane) {
+    if constexpr (ROLLED) {
+        constexpr int G = (N + 7) / 8;
+        float v[G * 8];
 #pragma unroll
-        for (int w = 0; w < NT / 32; w++) t += sm.red[w][0];
-        sm.tot[0] = t;
+        for (int q = 0; q < G * 8; q++) v[q] = q < N ? a[q] : 0.f;
+#pragma unroll 1
+        for (int g = 0; g < G; g++) {
+            __syncwarp();  // the buffer's last reader is done
+#pragma unroll
+            for (int j = 0; j < 8; j++) buf[lane * kBufPitch + j] = v[g * 8 + j];
+            __syncwarp();
+            column_sums(buf, dst + g * 8, min(8, N - g * 8), lane);
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < N; g += 8) {
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8 && g + j < N; j++) buf[lane * kBufPitch + j] = a[g + j];
+            __syncwarp();
+            column_sums(buf, dst + g, min(8, N - g), lane);
+        }
     }
-    __syncthreads();
-    const double t = sm.tot[0];
-    __syncthreads();
-    return t;
 }
 
-// The quintic basis at fraction t as symmetric pairs W[k] = (w_k, w_{5-k}),
-// k = 0..2: the weights of basis() split about t = 1/2 into an even part
-// e_k(v) and an odd part -u P_k(v) (u = t - 1/2, v = u^2), w_k = e_k - u P_k
-// and w_{5-k} = e_k + u P_k, each one FMA (the odd part is never rounded on
-// its own), in scalar FP32 ops whose polynomial coefficients are
-// instruction immediates; each weight lands in its half of the pair.
-__device__ __forceinline__ void basis_sym1(float t, float2 W[3]) {
-    const float u = t - 0.5f;
+// 1.5 x 2^23: adding it rounds an FP32 value of magnitude below 2^22 to an
+// integer, which then stands in the sum's low mantissa bits (offset by kMagic's
+// own bits, the bias that the window offsets take off again).
+constexpr float kMagic = 12582912.0f;
+constexpr uint32_t kMagicBits = 0x4B400000u;
+
+// The quintic basis at u = fraction - 1/2 as symmetric pairs W[k] = (w_k,
+// w_{5-k}), k = 0..2: the weights of basis() split into an even part
+// e_k(v) and an odd part -u q_k(v), v = u^2, w_k = e_k - u q_k and
+// w_{5-k} = e_k + u q_k, each one FMA (the odd part is never rounded on its
+// own), in scalar FP32 ops whose polynomial coefficients are instruction
+// immediates (as paired ops the coefficients take 18 registers, which the
+// sample loop does not have: 53 M sectors of spills on 8,836 second-order
+// subsets, 1.46 against 1.33 ms).
+__device__ __forceinline__ void basis_sym(float u, float2 W[3]) {
     const float v = u * u;
     const float e0 = fmaf(fmaf(v, 1.0f / 48.0f, 1.0f / 96.0f), v, 1.0f / 3840.0f);
     const float e1 = fmaf(fmaf(v, -1.0f / 16.0f, 7.0f / 32.0f), v, 79.0f / 1280.0f);
@@ -151,6 +194,13 @@ __device__ __forceinline__ void basis_sym1(float t, float2 W[3]) {
     W[0] = make_float2(fmaf(-u, q0, e0), fmaf(u, q0, e0));
     W[1] = make_float2(fmaf(-u, q1, e1), fmaf(u, q1, e1));
     W[2] = make_float2(fmaf(-u, q2, e2), fmaf(u, q2, e2));
+}
+
+// A record, read once per iteration: not kept in L1.
+__device__ __forceinline__ float4 ld_rec(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 
 // One coefficient row against the column weights: sum_k b_k c_k with the
@@ -193,7 +243,7 @@ struct KSum {
 // the cross term) go straight into the thread's compensated FP64 sums ks
 // instead of the run's FP32 partials.
 template <int ORDER, bool KAHAN>
-__device__ __forceinline__ void acc_sample(RunAcc &a, KSum (&ks)[3], float4 rec, float g, float fmf, float dyf) {
+__device__ __forceinline__ void acc_sample(RunAcc &a, KSum (&ks)[3], float4 rec, float g, float fmf, float2 dy2, float2 dd2) {
     const float gc = (g - fmf) * rec.w;
     if (KAHAN) {
         const double gd = (double)gc;
@@ -207,11 +257,8 @@ __device__ __forceinline__ void acc_sample(RunAcc &a, KSum (&ks)[3], float4 rec,
     }
     const float2 gxy = __fmul2_rn(make_float2(rec.x, rec.y), make_float2(gc, gc));
     a.m0 = __fadd2_rn(a.m0, gxy);
-    if (ORDER >= 1) a.m1 = __ffma2_rn(gxy, make_float2(dyf, dyf), a.m1);
-    if (ORDER == 2) {
-        const float d2 = dyf * dyf;
-        a.m2 = __ffma2_rn(gxy, make_float2(d2, d2), a.m2);
-    }
+    if (ORDER >= 1) a.m1 = __ffma2_rn(gxy, dy2, a.m1);
+    if (ORDER == 2) a.m2 = __ffma2_rn(gxy, dd2, a.m2);
 }
 
 // The run's steepest-descent sums into the thread's totals PB[mu] (pairs
@@ -231,7 +278,73 @@ __device__ __forceinline__ void acc_expand(const RunAcc &a, float dxf, float2 (&
     }
 }
 
-template <int ORDER, int NT, int K, bool KAHAN>
+// Omitted-mode diagnostic at the last sampled warp: g sampled again into RSG
+// (the solve keeps no samples), then eta_two_pass.  Only kernels instantiated
+// for it hold it: inside every solve it cost 4 % in registers and code.
+// fms: s - f_m.
+template <int ORDER, int NT, int K>
+__device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, const float *__restrict__ g32, int64_t pitch32,
+                                     int w, int h, int B, const int2 *tasks, int T, const float4 *REC, float *RSG,
+                                     const int *RVM, double cx, double cy, double fms, double dn, double df, double gm,
+                                     double dg, double *eu, double *ev) {
+    constexpr int M = Ord<ORDER>::M;
+    const int tid = threadIdx.x;
+    const double *pprev = sm.pprev;
+    const double X0 = cx + pprev[0], Y0 = cy + pprev[1];
+    const double bxd = floor(X0), byd = floor(Y0);
+    const int wbx = (int)bxd, wby = (int)byd;
+    const double ox = X0 - bxd, oy = Y0 - byd;
+    const bool staged = sm.win_ok != 0;  // the window the last iteration sampled
+    const int gr0 = sm.win_r0, gc0 = sm.win_c0, gwh = sm.win_h, gww = sm.win_w, gP = sm.win_p;
+    // this thread's template pixels; the first walk samples g again
+    auto each = [&](auto first, auto fn) {
+#pragma unroll 1
+        for (int t = tid; t < T; t += NT) {
+            int dxi, dy0;
+            unpack_task(tasks[t], dxi, dy0);
+            const int vm = RVM[t];
+#pragma unroll 1
+            for (int j = 0; j < K; j++) {
+                if (!((vm >> j) & 1)) continue;
+                const int sl = j * T + t;
+                const double dx = dxi, dy = dy0 + j;
+                if constexpr (decltype(first)::value) {
+                    double lx = ox + dx, ly = oy + dy;
+                    if (ORDER >= 1) {
+                        lx += pprev[2] * dx + pprev[4] * dy;
+                        ly += pprev[3] * dx + pprev[5] * dy;
+                    }
+                    if (ORDER == 2) {
+                        lx += 0.5 * pprev[6 % M] * dx * dx + pprev[8 % M] * dx * dy + 0.5 * pprev[10 % M] * dy * dy;
+                        ly += 0.5 * pprev[7 % M] * dx * dx + pprev[9 % M] * dx * dy + 0.5 * pprev[11 % M] * dy * dy;
+                    }
+                    int ix, iy;
+                    float tx, ty;  // integer offsets added exactly, the small parts in FP32
+                    split_clamped(wbx + dxi, (float)(lx - dx), w, ix, tx);
+                    split_clamped(wby + dy0 + j, (float)(ly - dy), h, iy, ty);
+                    float a[6], b[6];
+                    basis(ty, a);
+                    basis(tx, b);
+                    if (staged) {
+                        const int wx = min(max(ix + B - 2 - gc0, 0), gww - 6), wy = min(max(iy + B - 2 - gr0, 0), gwh - 6);
+                        RSG[sl] = contract<float>(win + wy * gP + wx, gP, a, b);
+                    } else {
+                        RSG[sl] = contract<float>(g32 + (int64_t)(iy + B - 2) * pitch32 + (ix + B - 2), pitch32, a, b);
+                    }
+                }
+                const float4 rec = REC[sl];
+                fn((double)rec.z + fms, (double)rec.x, (double)rec.y, (double)RSG[sl] - gm, dx, dy);
+            }
+        }
+    };
+    auto red = [&](auto &v) { run_block_sums<NT>(v, sm.red2, sm.aug); };
+    double u, v;
+    eta_two_pass<ORDER>(dn, df, dg, each, red, u, v);
+    *eu = u;
+    *ev = v;
+}
+
+template <int ORDER, int NT, int K, bool KAHAN, bool ETA>
 __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, float *base, float *win,
                            RunSmem<NT / 32> &sm) {
     const KArgs &A = R.k;
@@ -260,17 +373,14 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         // +-1: an FP32 fraction can round up to the next integer
         const int xlo = max(0, min(bx - re - 1, A.w - 1)), xhi = max(0, min(bx + re + 1, A.w - 1));
         const int ylo = max(0, min(by - re - 1, A.h - 1)), yhi = max(0, min(by + re + 1, A.h - 1));
-        int r0, c0, wh, ww, pitch;
-        const bool ok = run_plan<32>(xlo, xhi, ylo, yhi, B, R.win_cap, r0, c0, wh, ww, pitch);
-        if (ok) run_stage<NT>(A.f32, A.pitch32, ch, r0, c0, wh, ww, pitch, win, 0);
-        if (tid == 0) {
-            sm.win_ok = 0;  // g must be staged before the iterations
-            sm.win_r0 = r0; sm.win_c0 = c0; sm.win_h = wh; sm.win_w = ww; sm.win_p = pitch;
-            sm.flag[2] = ok;
+        place_window<NT>(sm, A.f32, A.pitch32, ch, B, R.win_cap, xlo, xhi, ylo, yhi, win, 0);
+        if (tid < M) {
+            sm.p[tid] = d.p0[tid];
+            sm.pprev[tid] = d.p0[tid];
         }
         __syncthreads();
     }
-    const bool f_staged = sm.flag[2] != 0;
+    const bool f_staged = sm.win_ok != 0;
     const int fr0 = sm.win_r0, fc0 = sm.win_c0, fwh = sm.win_h, fww = sm.win_w, fP = sm.win_p;
     // interior: every run pixel sits at an integer offset from the centre
     // inside the image, so all share one fraction and one basis
@@ -375,6 +485,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                     pix1(v, val, vx, vy, dx, dy0 + j);
                 }
             } else {
+#pragma unroll 1
                 for (int j = 0; j < K; j++) {
                     const bool v = (vm >> j) & 1u;
                     int ix, iy;
@@ -398,7 +509,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             }
         }
     }
-    run_warp_sums<NVA>(acc, sm.red2[wid], lane);
+    run_warp_sums<NVA, (NVA > 16)>(acc, sm.part[wid], sm.red2[wid], lane);
     // ---- setup, pass 2: the Hessian's gradient moments ----------------------
     // sum g_p g_q dx^a dy^b (a + b <= 2 DEG) per run as powers of dy, then
     // expanded by the run's powers of dx; each thread re-reads its own records
@@ -441,7 +552,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                     for (int p = 0; p < 3; p++)
                         mom[p * NMOM + mom_idx(a, b)] = fmaf(xp[a], V[p][b], mom[p * NMOM + mom_idx(a, b)]);
         }
-        run_warp_sums<3 * NMOM>(mom, sm.red2[wid] + NVA, lane);
+        run_warp_sums<3 * NMOM, (NMOM > 1)>(mom, sm.part[wid], sm.red2[wid] + NVA, lane);
     }
     __syncthreads();
     constexpr int NV = NVA + 3 * NMOM;
@@ -470,7 +581,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             if (lane < 3 * NMOM) sm.mom[lane] = sm.aug[NVA + lane];
             if (lane + 32 < 3 * NMOM) sm.mom[lane + 32] = sm.aug[NVA + lane + 32];
             __syncwarp();
-            if (!hess_factor_regs<ORDER>(sm.mom, sm.L, sm.linv, sm.dsc, lane)) st = GPV_SINGULAR_H;
+            if (!hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane)) st = GPV_SINGULAR_H;
         }
         if (lane == 0) {
             sm.flag[0] = st;
@@ -479,24 +590,10 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             sm.misc[7] = sm.aug[3];
             sm.n_valid = n;
         }
-        if (lane < M) {
-            sm.p[lane] = d.p0[lane];
-            sm.pprev[lane] = d.p0[lane];
-        }
     } else {
         // stage g's window around the initial warp
-        int xlo, xhi, ylo, yhi, r0 = 0, c0 = 0, wh = 0, ww = 0, pitch = 0;
-        bool inside;
-        double p0[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) p0[k] = d.p0[k % M];
-        run_extent<ORDER>(p0, cx, cy, re, A.w, A.h, xlo, xhi, ylo, yhi, &inside);
-        const bool ok = run_plan<32>(xlo, xhi, ylo, yhi, B, R.win_cap, r0, c0, wh, ww, pitch);
-        if (ok) run_stage<NT>(A.g32, A.pitch32, ch, r0, c0, wh, ww, pitch, win, 32);
-        if (tid == 32) {
-            sm.win_ok = ok;
-            sm.win_r0 = r0; sm.win_c0 = c0; sm.win_h = wh; sm.win_w = ww; sm.win_p = pitch;
-        }
+        const int4 ext = run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h);
+        place_window<NT>(sm, A.g32, A.pitch32, ch, B, R.win_cap, ext.x & ~kInside, ext.y, ext.z, ext.w, win, 32);
     }
     __syncthreads();
     const int st0 = sm.flag[0];
@@ -516,7 +613,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         return;
     }
     // H^-1 by every thread (warp 0 reads it only after the first iteration's barrier)
-    hess_inverse_block<M, NT>(sm.L, sm.dsc, sm.Hi);
+    hess_inverse_block<M, NT>(sm.L, sm.dsc, sm.Hi, tid);
 
     // ---- ICGN iterations --------------------------------------------------
     const double size = sqrt(dn);
@@ -526,21 +623,12 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     double c_zncc = 0.0, c_znssd = 4.0, last_norm = 0.0, gm_last = 0.0, dg_last = 0.0;
     for (int it = 1; it <= A.max_iter; it++) {
         // (re)stage g's window when the warped square has left it
-        bool inside;
-        {
-            int xlo, xhi, ylo, yhi;
-            run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h, xlo, xhi, ylo, yhi, &inside);
-            if (!run_covers(sm, xlo, xhi, ylo, yhi, B)) {
-                int r0, c0, wh, ww, pitch;
-                const bool ok = run_plan<32>(xlo, xhi, ylo, yhi, B, R.win_cap, r0, c0, wh, ww, pitch);
-                __syncthreads();  // nobody still reads the old window
-                if (ok) run_stage<NT>(A.g32, A.pitch32, ch, r0, c0, wh, ww, pitch, win, 0);
-                if (tid == 0) {
-                    sm.win_ok = ok;
-                    sm.win_r0 = r0; sm.win_c0 = c0; sm.win_h = wh; sm.win_w = ww; sm.win_p = pitch;
-                }
-                __syncthreads();
-            }
+        const int4 ext = run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h);
+        const bool inside = ext.x & kInside;
+        if (!run_covers(sm, ext.x & ~kInside, ext.y, ext.z, ext.w, B)) {
+            __syncthreads();  // nobody still reads the old window (or its place)
+            place_window<NT>(sm, A.g32, A.pitch32, ch, B, R.win_cap, ext.x & ~kInside, ext.y, ext.z, ext.w, win, 0);
+            __syncthreads();
         }
         const bool staged = sm.win_ok != 0;
         const int gr0 = sm.win_r0, gc0 = sm.win_c0, gwh = sm.win_h, gww = sm.win_w, gP = sm.win_p;
@@ -563,7 +651,10 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         // ((y, x) pairs; |s| ~ the fraction plus the deformation over the
         // subset): s is rounded in FP32 at its own small magnitude, and the
         // integer offsets join its floor exactly.
-        const float2 O2 = make_float2(oy, ox), U1 = make_float2(vx, ux), U2 = make_float2(vy, uy);
+        // (half a pixel lower on the fast path, where floors come by rounding)
+        const float half = fast ? 0.5f : 0.f;
+        const uint32_t o0 = 0u - kMagicBits * ((uint32_t)gP + 1u);
+        const float2 O2 = make_float2(oy - half, ox - half), U1 = make_float2(vx, ux), U2 = make_float2(vy, uy);
         const float2 Q1 = make_float2(vxx, uxx), Q2 = make_float2(vxy, uxy), C2 = make_float2(vyy, uyy);
         double s1 = 0.0, s2 = 0.0, sfg = 0.0;
         KSum ks[3];
@@ -587,51 +678,52 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             ac.p1 = ac.p2 = ac.pfg = 0.f;
             ac.m0 = ac.m1 = ac.m2 = make_float2(0.f, 0.f);
             if (fast) {
-                // no edge clamp can apply and the window covers every tap:
-                // the 6 x 6 block rolls down the run in registers
+                // no edge clamp can apply and the window covers every tap: the
+                // block of coefficients rolls down the run in registers, two
+                // samples per pass of a rolled loop (seven rows held; the last
+                // five move up two places between passes)
                 float Rg[6][6];
-                int fxp = 0, fyp = 0;
-                // window position of the run's first pixel at zero small part
-                const float *rbase = win + (dy0 + wy0) * gP + (dx + wx0);
-                const float dy0f = (float)dy0;
+                int py = 0, px = 0;  // floors of the sample before (biased)
+                uint32_t off = o0 + (uint32_t)((dy0 + wy0) * gP + dx + wx0);
+                const float4 *rec = REC + t;
+                float2 dy2 = make_float2((float)dy0, (float)dy0);
 #pragma unroll
                 for (int j = 0; j < K; j++) {
-                    const float dyf = dy0f + (float)j;  // exact: small integers
+                    const float4 rc = ld_rec(rec);
                     float2 L = A2;
-                    if (ORDER >= 1) L = __ffma2_rn(B2, make_float2(dyf, dyf), L);
-                    if (ORDER == 2) L = __ffma2_rn(C2, make_float2(dyf * dyf, dyf * dyf), L);
-                    const float fly = floorf(L.x), flx = floorf(L.y);
-                    const int iy = (int)fly, ix = (int)flx;  // floor offsets of the small part
-                    const float2 tt = __fadd2_rn(L, make_float2(-fly, -flx));
-                    const float *rp = rbase + (j + iy) * gP + ix;
-                    if (j == 0) {
+                    const float2 dd2 = __fmul2_rn(dy2, dy2);
+                    if (ORDER >= 1) L = __ffma2_rn(B2, dy2, L);
+                    if (ORDER == 2) L = __ffma2_rn(C2, dd2, L);
+                    // L is half a pixel below the position: rounding to
+                    // nearest gives its floor, and u = fraction - 1/2
+                    const float2 Mg = __fadd2_rn(L, make_float2(kMagic, kMagic));
+                    const float2 u2 = __fadd2_rn(L, __ffma2_rn(Mg, make_float2(-1.f, -1.f), make_float2(kMagic, kMagic)));
+                    const int iy = __float_as_int(Mg.x), ix = __float_as_int(Mg.y);
+                    const float *rp = win + (int)(off + (uint32_t)iy * (uint32_t)gP + (uint32_t)ix);
+                    if (j == 0 || ix != px || iy != py) {  // the block did not move down one row: (re)load
 #pragma unroll
-                        for (int rr = 0; rr < 6; rr++)
+                        for (int rr = 0; rr < 5; rr++)
 #pragma unroll
-                            for (int k = 0; k < 6; k++) Rg[rr][k] = rp[rr * gP + k];
-                    } else {
-                        if (ix != fxp || iy != fyp) {  // the block did not move down one row: reload
-#pragma unroll
-                            for (int rr = 0; rr < 5; rr++)
-#pragma unroll
-                                for (int k = 0; k < 6; k++) Rg[(j + rr) % 6][k] = rp[rr * gP + k];
-                        }
-#pragma unroll
-                        for (int k = 0; k < 6; k++) Rg[(j + 5) % 6][k] = rp[5 * gP + k];
+                            for (int k = 0; k < 6; k++) Rg[(j + rr) % 6][k] = rp[rr * gP + k];
                     }
-                    fxp = ix;
-                    fyp = iy;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) Rg[(j + 5) % 6][k] = rp[5 * gP + k];
+                    py = iy;
+                    px = ix;
                     float2 Aw[3], Bw[3];
-                    basis_sym1(tt.x, Aw);
-                    basis_sym1(tt.y, Bw);
+                    basis_sym(u2.y, Bw);
                     float sr[6];
 #pragma unroll
                     for (int rr = 0; rr < 6; rr++) sr[rr] = row_dot(Rg[(j + rr) % 6], Bw);
+                    basis_sym(u2.x, Aw);
                     const float g = combine6(sr, Aw);
-                    const int sl = j * T + t;
-                    acc_sample<ORDER, KAHAN>(ac, ks, REC[sl], g, fmf, dyf);
+                    acc_sample<ORDER, KAHAN>(ac, ks, rc, g, fmf, dy2, dd2);
+                    rec += T;
+                    off += (uint32_t)gP;
+                    dy2 = __fadd2_rn(dy2, make_float2(1.f, 1.f));
                 }
             } else {
+#pragma unroll 1
                 for (int j = 0; j < K; j++) {
                     const float dyf = (float)(dy0 + j);
                     float2 L = A2;
@@ -652,7 +744,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                         g = contract<float>(A.g32 + (int64_t)(iy + B - 2) * A.pitch32 + (ix + B - 2), A.pitch32, a, b);
                     }
                     const int sl = j * T + t;
-                    acc_sample<ORDER, KAHAN>(ac, ks, REC[sl], g, fmf, dyf);
+                    acc_sample<ORDER, KAHAN>(ac, ks, REC[sl], g, fmf, make_float2(dyf, dyf), make_float2(dyf * dyf, dyf * dyf));
                 }
             }
             if (!KAHAN) {
@@ -666,19 +758,24 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         // adds them up and updates the warp; a second barrier publishes p
         constexpr int KR = 3 + M;
         {
-            double v[KR];
+            double v[3] = {s1, s2, sfg};
             if (KAHAN) {
-                s1 = ks[0].s;
-                s2 = ks[1].s;
-                sfg = ks[2].s;
+                v[0] = ks[0].s;
+                v[1] = ks[1].s;
+                v[2] = ks[2].s;
             }
-            v[0] = s1; v[1] = s2; v[2] = sfg;
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const double t = warp_sum(v[q]);
+                if (lane == q) sm.red[wid][q] = t;
+            }
+            float pb[M];
 #pragma unroll
             for (int j = 0; j < M / 2; j++) {
-                v[3 + 2 * j] = (double)PB[j].x;
-                v[4 + 2 * j] = (double)PB[j].y;
+                pb[2 * j] = PB[j].x;
+                pb[2 * j + 1] = PB[j].y;
             }
-            warp_sum_many<KR>(v, sm.red[wid], lane);
+            run_warp_sums<M, false>(pb, sm.part[wid], sm.red[wid] + 3, lane);
         }
         __syncthreads();
         if (wid == 0) {
@@ -692,11 +789,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             const double gmt = t0 * inv_dn;
             const double dg2 = t1 - t0 * gmt;
             const double dg2p = dg2 > 0.0 ? dg2 : 0.0;
-            const double dg = sqrt(dg2p);
             // sum (f - f_m)(g - g_m) = sum (f - f_m)(g - f_m) (sum (f - f_m) = 0)
             //                     = sum (f - s)(g - f_m) - (f_m - s) sum (g - f_m)
             const double sab = t2 - (fm - (double)shift) * t0;
             const double rdg = rsqrt(dg2p);  // 1 / delta_g: one reciprocal square root on the update's critical path
+            const double dg = dg2p > 0.0 ? dg2p * rdg : 0.0;
             const double znssd = 2.0 - 2.0 * sab * (inv_df * rdg);
             const double ratio = df * rdg;
             // lane j < M: grad_j = A_j - (df/dg)(B_j - g~_m S_j); B_j sits at lane 3 + j
@@ -720,6 +817,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 sm.dp[lane] = dpj;
                 sm.pprev[lane] = sm.p[lane];
             }
+            // convergence_norm (src/subset.rs:622-649), a term per lane
+            double nt = lane < M ? dpj * (lane < 2 ? 1.0 : (lane < 6 ? size : 0.5 * dn)) : 0.0;
+            nt *= nt;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) nt += __shfl_down_sync(0xffffffffu, nt, o);
             __syncwarp();
             if (lane == 0) {
                 double pn[12], dpl[12], pl[12];
@@ -742,7 +844,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                     for (int k = 0; k < M; k++) sm.p[k] = pn[k];
                 }
                 sm.flag[1] = ok;
-                sm.misc[1] = conv_norm<M>(dpl, size);
+                sm.misc[1] = sqrt(nt);
                 sm.misc[2] = gmt;
                 sm.misc[3] = dg;
                 sm.misc[4] = znssd;
@@ -768,51 +870,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
 
     // ---- eta diagnostic at the last sampled warp (optional) -----------------
     double eu = 0.0, ev = 0.0;
-    const bool want_eta = (A.flags & GPV_SOLVE_ETA) && iters > 0 && status == GPV_OK;
-    if (want_eta) {
-        const double *pprev = sm.pprev;
-        const double X0 = cx + pprev[0], Y0 = cy + pprev[1];
-        const double bxd = floor(X0), byd = floor(Y0);
-        const int wbx = (int)bxd, wby = (int)byd;
-        const double ox = X0 - bxd, oy = Y0 - byd;
-        for (int i = tid; i < NS; i += NT) {
-            const int t = i % T, j = i / T;
-            if (!((RVM[t] >> j) & 1)) continue;
-            int dxi, dy0;
-            unpack_task(tasks[t], dxi, dy0);
-            const double dx = dxi, dy = dy0 + j;
-            double lx = ox + dx, ly = oy + dy;
-            if (ORDER >= 1) {
-                lx += pprev[2] * dx + pprev[4] * dy;
-                ly += pprev[3] * dx + pprev[5] * dy;
-            }
-            if (ORDER == 2) {
-                lx += 0.5 * pprev[6 % M] * dx * dx + pprev[8 % M] * dx * dy + 0.5 * pprev[10 % M] * dy * dy;
-                ly += 0.5 * pprev[7 % M] * dx * dx + pprev[9 % M] * dx * dy + 0.5 * pprev[11 % M] * dy * dy;
-            }
-            int ix, iy;
-            float tx, ty;  // integer offsets added exactly, the small parts in FP32
-            split_clamped(wbx + dxi, (float)(lx - dx), A.w, ix, tx);
-            split_clamped(wby + dy0 + j, (float)(ly - dy), A.h, iy, ty);
-            float a[6], b[6];
-            basis(ty, a);
-            basis(tx, b);
-            RSG[i] = contract<float>(A.g32 + (int64_t)(iy + B - 2) * A.pitch32 + (ix + B - 2), A.pitch32, a, b);
-        }
-        __syncthreads();
-        auto load = [&](int i, double &f, double &gx, double &gy, double &g, double &dx, double &dy) -> bool {
-            const int t = i % T, j = i / T;
-            if (!((RVM[t] >> j) & 1)) return false;
-            int dxi, dy0;
-            unpack_task(tasks[t], dxi, dy0);
-            const float4 rec = REC[i];
-            f = (double)rec.z + (double)shift;
-            gx = rec.x; gy = rec.y; g = RSG[i];
-            dx = dxi; dy = dy0 + j;
-            return true;
-        };
-        auto red = [&](double v) { return run_block_sum<NT>(v, sm); };
-        eta_sums<ORDER>(NS, tid, NT, dn, fm, df, gm_last, dg_last, load, red, eu, ev);
+    const bool want_eta = ETA && iters > 0 && status == GPV_OK;
+    if constexpr (ETA) {
+        if (want_eta)
+            run_eta<ORDER, NT, K>(sm, win, A.g32, A.pitch32, A.w, A.h, B, tasks, T, REC, RSG, RVM, cx, cy, (double)shift - fm,
+                              dn, df, gm_last, dg_last, &eu, &ev);
     }
     if (tid == 0) {
         gpv_subset_result *o = A.out + idx;
@@ -860,7 +922,7 @@ __device__ int run_claim_slot(const RunArgs &R) {
 // PER_SUBSET: one block per subset with a claimed scratch slot (subsets
 // free SMs one at a time, for callers sharing the GPU); else a persistent
 // grid whose blocks take subsets of their segment from the queue.
-template <int ORDER, int NT, int K, bool PER_SUBSET, bool KAHAN>
+template <int ORDER, int NT, int K, bool PER_SUBSET, bool KAHAN, bool ETA>
 __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
     extern __shared__ float4 win4[];
     float *win = reinterpret_cast<float *>(win4);
@@ -884,7 +946,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
         if (d.radius < 1 || d.radius > A.max_radius) {
             if (threadIdx.x == 0) write_failed(A, idx, d, 12, GPV_INVALID_SUBSET, 0, 0.0, 0.0);
         } else {
-            run_subset<ORDER, NT, K, KAHAN>(R, idx, d, base, win, sm);
+            run_subset<ORDER, NT, K, KAHAN, ETA>(R, idx, d, base, win, sm);
         }
         __threadfence();  // every scratch access of the block is done before the slot is free
         __syncthreads();
@@ -907,54 +969,27 @@ __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
             if (threadIdx.x == 0) write_failed(A, idx, d, 12, GPV_INVALID_SUBSET, 0, 0.0, 0.0);
             continue;
         }
-        run_subset<ORDER, NT, K, KAHAN>(R, idx, d, base, win, sm);
+        run_subset<ORDER, NT, K, KAHAN, ETA>(R, idx, d, base, win, sm);
     }
 }
 
-template <int NT, int K, bool PS, bool KH>
+// Instantiations: every (threads, one block per subset, with or without the
+// diagnostic); the compensated-sum form on persistent grids of 128 or 256
+// threads only.
+template <int NT, bool PS, bool KH, bool ETA>
 const void *run_kernel_t(int order) {
-    return order == 2 ? (const void *)icgn_runs<2, NT, K, PS, KH>
-                      : (order == 1 ? (const void *)icgn_runs<1, NT, K, PS, KH> : (const void *)icgn_runs<0, NT, K, PS, KH>);
-}
-
-template <int NT, int K, bool PS, bool KH>
-void run_launch_t(int order, int blocks, size_t smem, cudaStream_t s, const RunArgs &R) {
-    if (order == 2) icgn_runs<2, NT, K, PS, KH><<<blocks, NT, smem, s>>>(R);
-    else if (order == 1) icgn_runs<1, NT, K, PS, KH><<<blocks, NT, smem, s>>>(R);
-    else icgn_runs<0, NT, K, PS, KH><<<blocks, NT, smem, s>>>(R);
-}
-
-template <int NT, bool PS, bool KH>
-const void *run_kernel_k(int order, int K) {
-    return K == 4 ? run_kernel_t<NT, 4, PS, KH>(order) : run_kernel_t<NT, 8, PS, KH>(order);
-}
-
-template <int NT, bool PS, bool KH>
-void run_launch_k(int order, int K, int blocks, size_t smem, cudaStream_t s, const RunArgs &R) {
-    if (K == 4) run_launch_t<NT, 4, PS, KH>(order, blocks, smem, s, R);
-    else run_launch_t<NT, 8, PS, KH>(order, blocks, smem, s, R);
-}
-
-// Instantiations: every (threads, run length, one block per subset); the
-// compensated-sum form on persistent grids of 128 or 256 threads only.
-template <int NT>
-const void *run_kernel_nt(int order, int K, bool ps, bool kahan) {
-    if constexpr (NT >= 128) {
-        if (kahan) return run_kernel_k<NT, false, true>(order, K);
-    }
-    return ps ? run_kernel_k<NT, true, false>(order, K) : run_kernel_k<NT, false, false>(order, K);
+    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, PS, KH, ETA>
+                      : (order == 1 ? (const void *)icgn_runs<1, NT, kRunK, PS, KH, ETA>
+                                    : (const void *)icgn_runs<0, NT, kRunK, PS, KH, ETA>);
 }
 
 template <int NT>
-void run_launch_nt(int order, int K, bool ps, bool kahan, int blocks, size_t smem, cudaStream_t s, const RunArgs &R) {
+const void *run_kernel_nt(int order, bool ps, bool kahan, bool eta) {
     if constexpr (NT >= 128) {
-        if (kahan) {
-            run_launch_k<NT, false, true>(order, K, blocks, smem, s, R);
-            return;
-        }
+        if (kahan) return eta ? run_kernel_t<NT, false, true, true>(order) : run_kernel_t<NT, false, true, false>(order);
     }
-    if (ps) run_launch_k<NT, true, false>(order, K, blocks, smem, s, R);
-    else run_launch_k<NT, false, false>(order, K, blocks, smem, s, R);
+    if (ps) return eta ? run_kernel_t<NT, true, false, true>(order) : run_kernel_t<NT, true, false, false>(order);
+    return eta ? run_kernel_t<NT, false, false, true>(order) : run_kernel_t<NT, false, false, false>(order);
 }
 
 }  // namespace
@@ -963,96 +998,85 @@ void run_launch_nt(int order, int K, bool ps, bool kahan, int blocks, size_t sme
 // Host side: run tables, sizes and launches (called by the batched launcher).
 // ---------------------------------------------------------------------------
 
-// Task tables for run lengths 4 and 8 and radii 1..max_radius: per task
-// {dx (low 16 bits) | dy0 (high 16 bits), circle bits}, bands of K rows from
-// dy = -r, the last band moved up to end at dy = r (its rows already in the
-// band above masked off); columns [-w, w] with w the widest circle row of
-// the band.
+// Run tables for radii 1..max_radius: per run {dx (low 16 bits) | dy0 (high
+// 16 bits), circle bits}, bands of kRunK rows from dy = -r, the last band
+// moved up to end at dy = r (its rows already in the band above masked off);
+// columns [-w, w] with w the widest circle row of the band.
 int ensure_run_tables(gpv_context *ctx, int max_radius) {
     if (max_radius <= ctx->run_table_radius) return GPV_SUCCESS;
     const int R1 = max_radius + 1;
     std::vector<int32_t> tab;  // pairs
-    std::vector<int32_t> off(2 * R1, 0), cnt(2 * R1, 0);
-    for (int kk = 0; kk < 2; kk++) {
-        const int K = kRunLengths[kk];
-        for (int r = 1; r <= max_radius; r++) {
-            off[kk * R1 + r] = (int32_t)(tab.size() / 2);
-            int n = 0;
-            for (int b0 = -r; b0 <= r; b0 += K) {
-                const int dy0 = (2 * r + 1 >= K) ? std::min(b0, r - K + 1) : -r;
-                int w = -1;
-                for (int j = 0; j < K; j++) {
-                    const int y = dy0 + j;
-                    if (y < b0 || y > r) continue;
-                    // the row's exact integer half-width, then the band's widest
-                    int h = (int)std::floor(std::sqrt((double)(r * r - y * y)));
-                    while ((h + 1) * (h + 1) + y * y <= r * r) h++;
-                    while (h > 0 && h * h + y * y > r * r) h--;
-                    w = std::max(w, h);
-                }
-                for (int dx = -w; dx <= w; dx++) {
-                    uint32_t bits = 0;
-                    for (int j = 0; j < K; j++) {
-                        const int y = dy0 + j;
-                        if (y >= b0 && y <= r && dx * dx + y * y <= r * r) bits |= 1u << j;
-                    }
-                    tab.push_back((int32_t)((uint32_t)(dx & 0xffff) | ((uint32_t)dy0 << 16)));
-                    tab.push_back((int32_t)bits);
-                    n++;
-                }
+    std::vector<int32_t> off(R1, 0), cnt(R1, 0);
+    for (int r = 1; r <= max_radius; r++) {
+        off[r] = (int32_t)(tab.size() / 2);
+        int n = 0;
+        for (int b0 = -r; b0 <= r; b0 += kRunK) {
+            const int dy0 = (2 * r + 1 >= kRunK) ? std::min(b0, r - kRunK + 1) : -r;
+            int w = -1;
+            for (int j = 0; j < kRunK; j++) {
+                const int y = dy0 + j;
+                if (y < b0 || y > r) continue;
+                // the row's exact integer half-width, then the band's widest
+                int h = (int)std::floor(std::sqrt((double)(r * r - y * y)));
+                while ((h + 1) * (h + 1) + y * y <= r * r) h++;
+                while (h > 0 && h * h + y * y > r * r) h--;
+                w = std::max(w, h);
             }
-            cnt[kk * R1 + r] = n;
+            for (int dx = -w; dx <= w; dx++) {
+                uint32_t bits = 0;
+                for (int j = 0; j < kRunK; j++) {
+                    const int y = dy0 + j;
+                    if (y >= b0 && y <= r && dx * dx + y * y <= r * r) bits |= 1u << j;
+                }
+                tab.push_back((int32_t)((uint32_t)(dx & 0xffff) | ((uint32_t)dy0 << 16)));
+                tab.push_back((int32_t)bits);
+                n++;
+            }
         }
+        cnt[r] = n;
     }
-    if (int rc = ctx->run_tasks.ensure(tab.size() * sizeof(int32_t))) return rc;
-    if (int rc = ctx->run_off.ensure(off.size() * sizeof(int32_t))) return rc;
-    if (int rc = ctx->run_n.ensure(cnt.size() * sizeof(int32_t))) return rc;
-    GPV_CUDA_TRY(cudaMemcpy(ctx->run_tasks.ptr, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    GPV_CUDA_TRY(cudaMemcpy(ctx->run_off.ptr, off.data(), off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    GPV_CUDA_TRY(cudaMemcpy(ctx->run_n.ptr, cnt.data(), cnt.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    // one buffer, one copy: run offsets, run counts, runs (8-byte aligned)
+    std::vector<int32_t> all(off);
+    all.insert(all.end(), cnt.begin(), cnt.end());
+    all.insert(all.end(), tab.begin(), tab.end());
+    if (int rc = ctx->run_tab.ensure(all.size() * sizeof(int32_t))) return rc;
+    GPV_CUDA_TRY(cudaMemcpy(ctx->run_tab.ptr, all.data(), all.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     ctx->h_run_n = cnt;
     ctx->run_table_radius = max_radius;
     return GPV_SUCCESS;
 }
 
-int run_length_index(int K) { return K == kRunLengths[0] ? 0 : 1; }
-
 // Window capacity (floats) of a launch for subsets up to radius rmax: the
-// square of half side max(rmax, K - 1 - rmax) stretched by 6%, taps and
+// square of half side max(rmax, kRunK - 1 - rmax) stretched by 6%, taps and
 // margins, at a pitch of whole 32-float rows.
-int run_window_cap(int rmax, int K) {
-    const int e = std::max(rmax, K - 1 - rmax);
+int run_window_cap(int rmax) {
+    const int e = std::max(rmax, kRunK - 1 - rmax);
     const int rw = (int)std::ceil(1.06 * e) + 2;
     const int side = 2 * rw + 6 + 2 * kRunMargin + 4;
     return side * run_pitch<32>(side);
 }
 
-// Record slots per block (largest radius's tasks x K, rounded to 32) and the
+// Record slots per block (largest radius's runs x kRunK, rounded to 32) and the
 // scratch floats per block: a float4 record and an eta resample per slot +
 // one validity word per task.
-int64_t run_scratch_floats(gpv_context *ctx, int rmax, int K, int *nslot) {
-    const int R1 = ctx->run_table_radius + 1;
+int64_t run_scratch_floats(gpv_context *ctx, int rmax, int *nslot) {
     int T = 0;  // the most tasks of any radius up to rmax (the count is not monotone in r)
-    for (int r = 1; r <= rmax; r++) T = std::max(T, (int)ctx->h_run_n[run_length_index(K) * R1 + r]);
-    const int ns = (T * K + 31) / 32 * 32;
+    for (int r = 1; r <= rmax; r++) T = std::max(T, (int)ctx->h_run_n[r]);
+    const int ns = (T * kRunK + 31) / 32 * 32;
     *nslot = ns;
     return 5 * (int64_t)ns + (T + 31) / 32 * 32;
 }
 
-const void *run_kernel(int order, int nt, int K, bool per_subset, bool kahan) {
-    if (nt == 64) return run_kernel_nt<64>(order, K, per_subset, kahan);
-    return nt == 256 ? run_kernel_nt<256>(order, K, per_subset, kahan) : run_kernel_nt<128>(order, K, per_subset, kahan);
+const void *run_kernel(int order, int nt, bool per_subset, bool kahan, bool eta) {
+    if (nt == 64) return run_kernel_nt<64>(order, per_subset, kahan, eta);
+    return nt == 256 ? run_kernel_nt<256>(order, per_subset, kahan, eta) : run_kernel_nt<128>(order, per_subset, kahan, eta);
 }
 
-int run_launch(gpv_context *ctx, int order, int nt, int K, bool kahan, int blocks, size_t smem, cudaStream_t s,
-               const KArgs &k, const int32_t *seg, int *queue, int win_cap, int nslot, uint32_t *slot_mask,
-               int slots_per_sm, int n_mask) {
+int run_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,
+               const int32_t *seg, int *queue, int win_cap, int nslot, uint32_t *slot_mask, int slots_per_sm, int n_mask) {
     RunArgs R;
     R.k = k;
-    const int R1 = ctx->run_table_radius + 1, kk = run_length_index(K);
-    R.tasks = static_cast<const int2 *>(ctx->run_tasks.ptr);
-    R.task_off = static_cast<const int32_t *>(ctx->run_off.ptr) + kk * R1;
-    R.task_n = static_cast<const int32_t *>(ctx->run_n.ptr) + kk * R1;
+    run_tables(ctx, R);
     R.seg = seg;
     R.queue = queue;
     R.win_cap = win_cap;
@@ -1060,15 +1084,8 @@ int run_launch(gpv_context *ctx, int order, int nt, int K, bool kahan, int block
     R.slot_mask = slot_mask;
     R.slots_per_sm = slots_per_sm;
     R.n_mask = n_mask;
-    const bool ps = slot_mask != nullptr;
-    if (kahan && (ps || nt == 64)) {
-        set_error("the compensated-sum form runs on persistent grids of 128 or 256 threads");
-        return GPV_ERR_INVALID;
-    }
-    if (nt == 64) run_launch_nt<64>(order, K, ps, kahan, blocks, smem, s, R);
-    else if (nt == 256) run_launch_nt<256>(order, K, ps, kahan, blocks, smem, s, R);
-    else run_launch_nt<128>(order, K, ps, kahan, blocks, smem, s, R);
-    GPV_CUDA_TRY(cudaGetLastError());
+    void *args[] = {&R};
+    GPV_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3((unsigned)nt), args, smem, s));
     return GPV_SUCCESS;
 }
 

@@ -29,7 +29,7 @@
 //  * FAGN takes two sweeps: target value and gradient at the warped positions
 //    (kept per pixel), then the Hessian's moments and the residual gradient
 //    about the warped centre.
-//  * The Hessian is factored by one warp (hess_factor_regs); a matrix that the
+//  * The Hessian is factored by one warp (hess_factor); a matrix that the
 //    factor rejects goes to the pivoted elimination (gj_inverse), so only what
 //    that rejects is singular.  Second-order composition eliminates without
 //    pivoting while the pivots stay near 1, else with pivoting.
@@ -48,13 +48,13 @@
 namespace gpv {
 namespace {
 
-constexpr int kK = 4;  // template pixels per run
+constexpr int kK = kRunK;
 
 template <int NW>
 struct Smem64 {
     double mom[3 * 15];
     double L[144];   // the factor's inverse
-    double Hi[144];  // H^-1
+    double Hi[160];  // the factor, then H^-1
     double linv[12], dsc[12];
     double A[12], S[12];
     double p[12], pprev[12], dp[12], grad[12];
@@ -94,19 +94,6 @@ __device__ __forceinline__ void stage64(const C *__restrict__ coef, int64_t cpit
         }
     }
     if (V == 2) asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-// Warp sums of KV values into dst[0..KV), 16 at a time.
-template <int KV, int C = 0>
-__device__ __forceinline__ void warp_sums64(const double (&a)[KV], double *dst, int lane) {
-    if constexpr (C < KV) {
-        constexpr int N = (KV - C) < 16 ? (KV - C) : 16;
-        double v[N];
-#pragma unroll
-        for (int j = 0; j < N; j++) v[j] = a[C + j];
-        warp_sum_many<N>(v, dst + C, lane);
-        warp_sums64<KV, C + N>(a, dst, lane);
-    }
 }
 
 template <int NT>
@@ -225,6 +212,10 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             sm.win_ok = 0;
             sm.win_r0 = r0; sm.win_c0 = c0; sm.win_h = wh; sm.win_w = ww; sm.win_p = pitch;
             sm.flag[2] = ok;
+        }
+        if (tid < M) {
+            sm.p[tid] = d.p0[tid];
+            sm.pprev[tid] = d.p0[tid];
         }
         __syncthreads();
     }
@@ -386,7 +377,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             }
             for (int q = lane; q < 3 * NMOM; q += 32) sm.mom[q] = sm.tot[NVA + q];
             __syncwarp();
-            const bool ok = hess_factor_regs<ORDER>(sm.mom, sm.L, sm.linv, sm.dsc, lane);
+            const bool ok = hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane);
             if (!ok) {
                 assemble_hessian<ORDER>(sm.mom, sm.L, lane);
                 int g = 0;
@@ -403,18 +394,10 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             sm.misc[8] = ms;
             sm.n_valid = n;
         }
-        if (lane < M) {
-            sm.p[lane] = d.p0[lane];
-            sm.pprev[lane] = d.p0[lane];
-        }
     } else {
-        int xlo, xhi, ylo, yhi, r0 = 0, c0 = 0, wh = 0, ww = 0, pitch = 0;
-        bool inside;
-        double p0[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) p0[k] = d.p0[k % M];
-        run_extent<ORDER>(p0, cx, cy, re, A.w, A.h, xlo, xhi, ylo, yhi, &inside);
-        const bool ok = run_plan<16>(xlo, xhi, ylo, yhi, B, R.win_cap, r0, c0, wh, ww, pitch);
+        int r0 = 0, c0 = 0, wh = 0, ww = 0, pitch = 0;
+        const int4 ext = run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h);
+        const bool ok = run_plan<16>(ext.x & ~kInside, ext.y, ext.z, ext.w, B, R.win_cap, r0, c0, wh, ww, pitch);
         if (ok) stage64<NT>(GC, cp, ch, r0, c0, wh, ww, pitch, win, 32);
         if (tid == 32) {
             sm.win_ok = ok;
@@ -436,7 +419,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         return;
     }
     // read by warp 0 only after the first iteration's barrier
-    if (!FAGN && sm.flag[3]) hess_inverse_block<M, NT>(sm.L, sm.dsc, sm.Hi);
+    if (!FAGN && sm.flag[3]) hess_inverse_block<M, NT>(sm.L, sm.dsc, sm.Hi, tid);
 
     // ---- iterations ---------------------------------------------------------
     const double size = sqrt(dn);
@@ -448,8 +431,9 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
     for (int it = 1; it <= A.max_iter; it++) {
         bool inside;
         {
-            int xlo, xhi, ylo, yhi;
-            run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h, xlo, xhi, ylo, yhi, &inside);
+            const int4 ext = run_extent<ORDER>(sm.p, cx, cy, re, A.w, A.h);
+            inside = ext.x & kInside;
+            const int xlo = ext.x & ~kInside, xhi = ext.y, ylo = ext.z, yhi = ext.w;
             if (!run_covers(sm, xlo, xhi, ylo, yhi, B)) {
                 int r0, c0, wh, ww, pitch;
                 const bool ok = run_plan<16>(xlo, xhi, ylo, yhi, B, R.win_cap, r0, c0, wh, ww, pitch);
@@ -681,7 +665,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 __syncwarp();
                 znssd = sm.tot[M];
                 // dp = H^-1 grad by the factor's inverse: D L^-T (L^-1 (D grad))
-                if (hess_factor_regs<ORDER>(sm.mom, sm.L, sm.linv, sm.dsc, lane)) {
+                if (hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane)) {
                     double y = 0.0;
                     if (lane < M) {
 #pragma unroll
@@ -794,50 +778,48 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
     double eu = 0.0, ev = 0.0;
     const bool want_eta = (A.flags & GPV_SOLVE_ETA) && iters > 0 && status == GPV_OK;
     if (want_eta) {
-        if constexpr (!FAGN) {
-            const double *pp = sm.pprev;
-            const double X0 = cx + pp[0], Y0 = cy + pp[1];
-            const double bxd = floor(X0), byd = floor(Y0);
-            const int wbx = (int)bxd, wby = (int)byd;
-            for (int i = tid; i < NS; i += NT) {
-                const int t = i % T, j = i / T;
-                if (!((RVM[t] >> j) & 1)) continue;
+        const double *pp = sm.pprev;
+        const double X0 = cx + pp[0], Y0 = cy + pp[1];
+        const double bxd = floor(X0), byd = floor(Y0);
+        const int wbx = (int)bxd, wby = (int)byd;
+        // this thread's template pixels; the first walk (FIRST) samples g again where the solve kept none
+        auto each = [&](auto first, auto fn) {
+#pragma unroll 1
+            for (int t = tid; t < T; t += NT) {
                 int dxi, dy0;
                 unpack_task(tasks[t], dxi, dy0);
-                const double dx = dxi, dy = dy0 + j;
-                double lx = X0 - bxd, ly = Y0 - byd;
-                if (ORDER >= 1) {
-                    lx += pp[2 % M] * dx + pp[4 % M] * dy;
-                    ly += pp[3 % M] * dx + pp[5 % M] * dy;
+                const int vm = RVM[t];
+#pragma unroll 1
+                for (int j = 0; j < kK; j++) {
+                    if (!((vm >> j) & 1)) continue;
+                    const int sl = j * T + t;
+                    const double dx = dxi, dy = dy0 + j;
+                    if constexpr (!FAGN && decltype(first)::value) {
+                        double lx = X0 - bxd, ly = Y0 - byd;
+                        if (ORDER >= 1) {
+                            lx += pp[2 % M] * dx + pp[4 % M] * dy;
+                            ly += pp[3 % M] * dx + pp[5 % M] * dy;
+                        }
+                        if (ORDER == 2) {
+                            lx += 0.5 * pp[6 % M] * dx * dx + pp[8 % M] * dx * dy + 0.5 * pp[10 % M] * dy * dy;
+                            ly += 0.5 * pp[7 % M] * dx * dx + pp[9 % M] * dx * dy + 0.5 * pp[11 % M] * dy * dy;
+                        }
+                        int ix, iy;
+                        double tx, ty;
+                        split_clamped(wbx + dxi, lx, A.w, ix, tx);
+                        split_clamped(wby + dy0 + j, ly, A.h, iy, ty);
+                        double a[6], b[6];
+                        basis(ty, a);
+                        basis(tx, b);
+                        RT[sl] = contract<double>(GC + (int64_t)(iy + B - 2) * cp + (ix + B - 2), cp, a, b);
+                    }
+                    const double2 q = RG[sl];
+                    fn(RF[sl] - fms, q.x, q.y, RT[sl] - gm_last, dx, dy);
                 }
-                if (ORDER == 2) {
-                    lx += 0.5 * pp[6 % M] * dx * dx + pp[8 % M] * dx * dy + 0.5 * pp[10 % M] * dy * dy;
-                    ly += 0.5 * pp[7 % M] * dx * dx + pp[9 % M] * dx * dy + 0.5 * pp[11 % M] * dy * dy;
-                }
-                int ix, iy;
-                double tx, ty;
-                split_clamped(wbx + dxi, lx, A.w, ix, tx);
-                split_clamped(wby + dy0 + j, ly, A.h, iy, ty);
-                double a[6], b[6];
-                basis(ty, a);
-                basis(tx, b);
-                RT[i] = contract<double>(GC + (int64_t)(iy + B - 2) * cp + (ix + B - 2), cp, a, b);
             }
-        }
-        __syncthreads();
-        auto load = [&](int i, double &f, double &gx, double &gy, double &g, double &dx, double &dy) -> bool {
-            const int t = i % T, j = i / T;
-            if (!((RVM[t] >> j) & 1)) return false;
-            int dxi, dy0;
-            unpack_task(tasks[t], dxi, dy0);
-            const double2 q = RG[i];
-            f = RF[i] + shift;
-            gx = q.x; gy = q.y; g = RT[i];
-            dx = dxi; dy = dy0 + j;
-            return true;
         };
-        auto red = [&](double v) { return block_sum64<NT>(v, sm); };
-        eta_sums<ORDER>(NS, tid, NT, dn, fm, df, gm_last, dg_last, load, red, eu, ev);
+        auto red = [&](auto &v) { run_block_sums<NT>(v, sm.red2, sm.tot); };
+        eta_two_pass<ORDER>(dn, df, dg_last, each, red, eu, ev);
     }
     if (tid == 0) {
         gpv_subset_result *o = A.out + idx;
@@ -897,8 +879,6 @@ const void *kernel64_nt(int order, bool fagn, bool c64) {
 
 }  // namespace
 
-int run64_run_length() { return kK; }
-
 // Window capacity (doubles): as run_window_cap, at the FP64 pitch.
 int run64_window_cap(int rmax) {
     const int e = std::max(rmax, kK - 1 - rmax);
@@ -921,10 +901,7 @@ int run64_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t sm
                  const int32_t *seg, int *queue, int win_cap, int nslot) {
     RunArgs R;
     R.k = k;
-    const int R1 = ctx->run_table_radius + 1, kk = run_length_index(kK);
-    R.tasks = static_cast<const int2 *>(ctx->run_tasks.ptr);
-    R.task_off = static_cast<const int32_t *>(ctx->run_off.ptr) + kk * R1;
-    R.task_n = static_cast<const int32_t *>(ctx->run_n.ptr) + kk * R1;
+    run_tables(ctx, R);
     R.seg = seg;
     R.queue = queue;
     R.win_cap = win_cap;

@@ -1307,8 +1307,8 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
     struct Plan {
         int rmax = 0, nt = 0, layout = 0, cap = 0, blocks = 0, per_sm = 0;
         bool ps = false, rigid = false;  // one block per subset; rigid-texture template
-        bool runs = false;               // the run-layout kernel (icgn_runs.cu), run length run_k
-        int run_k = 0, nslot = 0;
+        bool runs = false;               // the run-layout kernel (icgn_runs.cu)
+        int nslot = 0;
         int64_t stride = 0;
         size_t smem = 0;                 // window bytes
         const void *fn = nullptr;
@@ -1333,7 +1333,6 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             // FP64 run layout: 3 blocks of 128 threads per SM up to radius 32 (the
             // windows of three blocks fit), 256 threads where fewer windows fit
             P.nt = P.rmax > 32 ? 256 : 128;
-            P.run_k = run64_run_length();
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
             P.fn = run64_kernel(order, P.nt, fagn, K.f64 != nullptr);
             int max_bytes = 0;
@@ -1342,7 +1341,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             P.smem = sizeof(double) * (size_t)P.cap;
             GPV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P.per_sm, P.fn, P.nt, P.smem));
             if (P.per_sm < 1) { set_error("subset window does not fit in shared memory"); return GPV_ERR_INVALID; }
-            run_scratch_floats(ctx, P.rmax, P.run_k, &P.nslot);
+            run_scratch_floats(ctx, P.rmax, &P.nslot);
             P.stride = 2 * run64_scratch_doubles(P.nslot, fagn);  // floats
             P.blocks = (int)std::min<int64_t>((int64_t)P.per_sm * ctx->num_sms, n);
             region = std::max(region, P.blocks * P.stride);
@@ -1358,13 +1357,14 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
         P.runs = !P.rigid && (use_run_kernel() || kahan);
         if (kahan) P.ps = false;
         if (P.runs) {
-            P.run_k = run_length_for(ctx, P.rmax);
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
         }
-        P.cap = P.runs ? run_window_cap(P.rmax, P.run_k) : window_cap(P.rmax, P.layout);
+        P.cap = P.runs ? run_window_cap(P.rmax) : window_cap(P.rmax, P.layout);
         // 64-thread blocks exist for the run-layout kernel (not its compensated form) only
         if (P.nt == 64 && (!P.runs || kahan)) P.nt = 128;
-        const void *fn = P.runs ? run_kernel(order, P.nt, P.run_k, P.ps, kahan) : tile_kernel(P.nt, P.ps, order, P.rigid);
+        const void *fn = P.runs ? run_kernel(order, P.nt, P.ps, kahan, (K.flags & GPV_SOLVE_ETA) != 0)
+                                : tile_kernel(P.nt, P.ps, order, P.rigid);
+        P.fn = fn;
         int max_bytes = 0;
         if (int rc = allow_max_dynamic_smem(fn, &max_bytes)) return rc;
         // a window larger than the block can hold is not staged: those
@@ -1391,7 +1391,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
         P.per_sm = per_sm;
         const int64_t nmax = (int64_t)(ctx->h_slot_n[P.rmax] + 31) / 32 * 32;
         P.stride = (P.rigid ? 9 : 5) * nmax;  // float4 record + eta sample (+ 3 grain samples, template) per pixel
-        if (P.runs) P.stride = run_scratch_floats(ctx, P.rmax, P.run_k, &P.nslot);
+        if (P.runs) P.stride = run_scratch_floats(ctx, P.rmax, &P.nslot);
         int64_t slots;
         if (P.ps) {
             P.blocks = (int)ctx->seg_count[q];
@@ -1440,9 +1440,8 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             T.k.scratch_stride = P.stride / 2;  // doubles
             if (int rc = run64_launch(ctx, P.fn, P.nt, P.blocks, P.smem, st[k], T.k, T.seg, T.queue, P.cap, P.nslot)) return rc;
         } else if (P.runs) {
-            if (int rc = run_launch(ctx, 2 - q / kRClasses, P.nt, P.run_k, (K.flags & GPV_SOLVE_KAHAN) != 0, P.blocks,
-                                    smem, st[k], T.k, T.seg, T.queue, P.cap, P.nslot, T.slot_mask, T.slots_per_sm,
-                                    T.n_mask))
+            if (int rc = run_launch(ctx, P.fn, P.nt, P.blocks, smem, st[k], T.k, T.seg, T.queue, P.cap, P.nslot, T.slot_mask,
+                                    T.slots_per_sm, T.n_mask))
                 return rc;
         } else {
             tile_launch_one(P.nt, P.ps, 2 - q / kRClasses, P.rigid, P.blocks, smem, st[k], T);
@@ -1474,14 +1473,6 @@ int tile_layout_for(gpv_context *ctx, int max_radius) {
 bool use_run_kernel() {
     const char *v = getenv("GPV_SOLVE_KERNEL");
     return !(v && v[0] == 't');
-}
-
-int run_length_for(gpv_context *ctx, int max_radius) {
-    if (ctx->force_run_k) return ctx->force_run_k;
-    if (const char *v = getenv("GPV_RUN_K")) return atoi(v) == 4 ? 4 : 8;
-    const int cls = max_radius <= 20 ? 0 : (max_radius <= 40 ? 1 : 2);
-    if (ctx->tuned_run_k[cls]) return ctx->tuned_run_k[cls];
-    return 4;
 }
 
 int tile_threads_for(gpv_context *ctx, int max_radius) {

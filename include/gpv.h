@@ -456,10 +456,9 @@ int gpv_server_destroy(gpv_server *s);
 
 /* ---- autotuning (no counterpart in the reference) ------------------------
  * Times the candidate launch shapes of the mixed-precision kernel (threads
- * per subset block: 64, 128 or 256; template pixels per run of the
- * run-layout kernel: 4 or 8 -- or, with GPV_SOLVE_KERNEL=tile, 128 or 256
- * threads and the tiled kernel's
- * template layout: compact scan order or 8 x 4 tiles) on a sample of up to
+ * per subset block: 64, 128 or 256 -- or, with GPV_SOLVE_KERNEL=tile, 128 or
+ * 256 threads and the tiled kernel's template layout: compact scan order or
+ * 8 x 4 tiles) on a sample of up to
  * sample_per_class subsets of each radius class
  * (r <= 20, 21..40, > 40) present in desc, keeps the fastest per class in the
  * context, and returns the thread choices in threads_out[3] (0 = class
@@ -477,7 +476,7 @@ int gpv_context_tuning(gpv_context *ctx, int32_t *threads, int32_t *layouts);
 typedef struct {
     int32_t threads;            /* threads per block: 64, 128 or 256                    */
     int32_t layout;             /* tiled kernel's template layout (-1, 0, 1, 2)         */
-    int32_t run_length;         /* run-layout kernel: template pixels per run, 4 or 8   */
+    int32_t run_length;         /* run-layout kernel: template pixels per run (4)       */
     int32_t subsets_per_block;  /* subsets a block solves side by side (1 or 2)         */
     int32_t staging;            /* coefficient-window buffers per subset (1 or 2)       */
     int32_t reserved;
