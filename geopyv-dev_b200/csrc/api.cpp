@@ -62,10 +62,11 @@ void HostBuf::release() {
     bytes = 0;
 }
 
-// Layout of the pinned staging of a host batch of n subsets: descriptors,
-// work order, results, each at a 256-byte boundary.
-static size_t stage_off_order(int64_t n) { return (sizeof(gpv_subset_desc) * (size_t)n + 255) / 256 * 256; }
-static size_t stage_off_out(int64_t n) { return stage_off_order(n) + (sizeof(int32_t) * (size_t)n + 255) / 256 * 256; }
+// Layout of the pinned staging of a host batch of n subsets: descriptors, the
+// launcher's segment table with the work order behind it (as tile_ws holds
+// them on the device), results, each at a 256-byte boundary.
+static size_t stage_off_ws(int64_t n) { return (sizeof(gpv_subset_desc) * (size_t)n + 255) / 256 * 256; }
+static size_t stage_off_out(int64_t n) { return stage_off_ws(n) + (sizeof(int32_t) * (kTileWs + (size_t)n) + 255) / 256 * 256; }
 static size_t stage_bytes(int64_t n) { return stage_off_out(n) + sizeof(gpv_subset_result) * (size_t)n; }
 
 int image_pixels_in(gpv_image *img, const void *px_dev, int dtype, cudaStream_t s, bool staged) {
@@ -288,7 +289,7 @@ static void context_release(gpv_context *ctx) {
     DeviceGuard dg(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (DevBuf *b : {&ctx->offs, &ctx->slots, &ctx->tab_off, &ctx->tab_n, &ctx->scratch, &ctx->queue, &ctx->desc_dev, &ctx->out_dev,
-                      &ctx->order_dev, &ctx->hist_dev, &ctx->eval_dev, &ctx->tile_ws, &ctx->slot_mask,
+                      &ctx->hist_dev, &ctx->eval_dev, &ctx->tile_ws, &ctx->slot_mask,
                       &ctx->run_tab})
         b->release();
     ctx->h_stage.release();
@@ -680,8 +681,7 @@ int gpv_context_reserve(gpv_context *ctx, int64_t n_subsets, int32_t max_radius,
     if (int rc = ctx->queue.ensure(64)) return rc;
     if (int rc = ctx->desc_dev.ensure(sizeof(gpv_subset_desc) * (size_t)n_subsets)) return rc;
     if (int rc = ctx->out_dev.ensure(sizeof(gpv_subset_result) * (size_t)n_subsets)) return rc;
-    if (int rc = ctx->order_dev.ensure(sizeof(int32_t) * (size_t)n_subsets)) return rc;
-    if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (96 + (size_t)n_subsets))) return rc;
+    if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (kTileWs + (size_t)n_subsets))) return rc;
     if (int rc = ctx->h_stage.ensure(stage_bytes(n_subsets))) return rc;
     (void)max_iterations;
     return GPV_SUCCESS;
@@ -721,12 +721,14 @@ int gpv_solve_batch(gpv_context *ctx, const gpv_image *f, const gpv_image *g, co
     // driver's own staging, which can wait behind other streams' work)
     if (int rc = ctx->h_stage.ensure(stage_bytes(n))) return rc;
     char *stage = static_cast<char *>(ctx->h_stage.ptr);
-    int32_t *order = reinterpret_cast<int32_t *>(stage + stage_off_order(n));
+    int32_t *ws = reinterpret_cast<int32_t *>(stage + stage_off_ws(n)), *order = ws + kTileWs;
     const size_t desc_bytes = sizeof(gpv_subset_desc) * (size_t)n, out_bytes = sizeof(gpv_subset_result) * (size_t)n;
-    const bool desc_pinned = host_pinned(desc, desc_bytes), out_pinned = host_pinned(out, out_bytes);
+    // (up to 256 KB a copy into the staging costs less than asking what memory it is)
+    const bool desc_pinned = desc_bytes > (256u << 10) && host_pinned(desc, desc_bytes);
+    const bool out_pinned = out_bytes > (256u << 10) && host_pinned(out, out_bytes);
     if (int rc = ctx->desc_dev.ensure(desc_bytes)) return rc;
     if (int rc = ctx->out_dev.ensure(out_bytes)) return rc;
-    if (int rc = ctx->order_dev.ensure(sizeof(int32_t) * n)) return rc;
+    if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (kTileWs + (size_t)n))) return rc;
     double *hist_dev = nullptr;
     const size_t hist_bytes = sizeof(double) * 3 * (size_t)n * (size_t)(prm->max_iterations > 0 ? prm->max_iterations : 1);
     if (prm->history) {
@@ -740,55 +742,64 @@ int gpv_solve_batch(gpv_context *ctx, const gpv_image *f, const gpv_image *g, co
     } else if (int rc = upload_staged(ctx->desc_dev.ptr, desc, stage, desc_bytes, ctx->stream)) {
         return rc;
     }
-    // largest subsets first (longest-processing-time order for the work
-    // queue): a counting sort on key = 3 * radius + order, larger radius
-    // first, order 2 before 1 before 0 (invalid subsets in bucket 0).  One
-    // pass builds the histogram and finds the largest radius; the segment
-    // sizes of the tiled launch come from the histogram.
-    constexpr int kMaxR = 4000;
-    constexpr int nk = 3 * (kMaxR + 1);
-    static_assert(nk <= 65536, "work-order keys are 16-bit");
-    std::vector<int64_t> start(nk + 1, 0);
+    // The work order by launch segment, larger radius classes first and larger
+    // radii first within a segment (longest-processing-time order for the work
+    // queues), in the form the partition kernels leave on the device: the launcher
+    // then needs neither them nor their clearing (12 us of a 75 us batch of
+    // tens of subsets).  Invalid subsets come last, in no segment.
+    constexpr int kMaxR = 4000, kInvalid = kTileSegs << 12;
     auto key = [](const gpv_subset_desc &d) -> int {
         const int r = d.radius, o = d.order;
-        if (r < 1 || r > kMaxR || o < 0 || o > 2) return 0;
-        return nk - 1 - (3 * r + o);
+        if (r < 1 || r > kMaxR || o < 0 || o > 2) return kInvalid;
+        const int q = tile_segment_of(r, o), rank = (3 - q % 4) * 3 + q / 4;
+        return (rank << 12) + (kMaxR - r);
     };
+    static_assert(kTileSegs == 12 && kMaxR < 4096 && kInvalid < 65536, "12 segments of 4096 keys, 16 bits");
     // the descriptors are read once: keys kept compact for the scatter
     ctx->h_keys.resize((size_t)n);
     uint16_t *keys = ctx->h_keys.data();
     int max_r = 1;
+    bool one_key = true;
+    for (int q = 0; q < kTileSegs; q++) ctx->seg_count[q] = 0;
+    int64_t invalid = 0;
     for (int64_t i = 0; i < n; i++) {
         const gpv_subset_desc &d = desc[i];
         const int k = key(d);
         keys[i] = (uint16_t)k;
-        start[k + 1]++;
+        one_key &= k == keys[0];
         if (d.radius > max_r && d.radius <= kMaxR) max_r = d.radius;
+        if (k == kInvalid) invalid++;
+        else ctx->seg_count[tile_segment_of(d.radius, d.order)]++;
     }
-    const bool one_key = start[keys[0] + 1] == n;  // every subset in one bucket: the order is 0..n-1
     if (int rc = ensure_tables(ctx, max_r)) return rc;
-    uint32_t seg_mask = 0;
-    for (int q = 0; q < kTileSegs; q++) ctx->seg_count[q] = 0;
-    for (int r = 1; r <= max_r; r++)
-        for (int o = 0; o <= 2; o++) {
-            const int64_t c = start[nk - 1 - (3 * r + o) + 1];
-            if (!c) continue;
-            const int q = tile_segment_of(r, o);
-            ctx->seg_count[q] += c;
-            seg_mask |= 1u << q;
-        }
     if (one_key) {
         for (int64_t i = 0; i < n; i++) order[i] = (int32_t)i;
+    } else if (n <= 4096) {
+        for (int64_t i = 0; i < n; i++) order[i] = (int32_t)i;
+        std::stable_sort(order, order + n, [&](int32_t a, int32_t b) { return keys[a] < keys[b]; });
     } else {
-        for (int k = 0; k < nk; k++) start[k + 1] += start[k];
+        std::vector<int32_t> start(kInvalid + 2, 0);
+        for (int64_t i = 0; i < n; i++) start[keys[i] + 1]++;
+        for (int k = 0; k <= kInvalid; k++) start[k + 1] += start[k];
         for (int64_t i = 0; i < n; i++) order[start[keys[i]]++] = (int32_t)i;
     }
-    GPV_CUDA_TRY(cudaMemcpyAsync(ctx->order_dev.ptr, order, sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx->stream));
+    std::memset(ws, 0, sizeof(int32_t) * kTileWs);
+    uint32_t seg_mask = 0;
+    int32_t at = 0;
+    for (int rank = 0; rank < kTileSegs; rank++) {
+        const int q = (rank % 3) * 4 + (3 - rank / 3);
+        ws[kTileWsSeg + 2 * q] = at;
+        ws[kTileWsSeg + 2 * q + 1] = (int32_t)ctx->seg_count[q];
+        at += (int32_t)ctx->seg_count[q];
+        if (ctx->seg_count[q]) seg_mask |= 1u << q;
+    }
+    GPV_CUDA_TRY(cudaMemcpyAsync(ctx->tile_ws.ptr, ws, sizeof(int32_t) * (kTileWs + (size_t)n), cudaMemcpyHostToDevice,
+                                 ctx->stream));
     SolveLaunch L;
     L.f = f;
     L.g = g;
     L.desc = static_cast<const gpv_subset_desc *>(ctx->desc_dev.ptr);
-    L.order = static_cast<const int32_t *>(ctx->order_dev.ptr);
+    L.order = static_cast<const int32_t *>(ctx->tile_ws.ptr) + kTileWs;
     L.n = n;
     L.prm = prm;
     L.mask = prm->mask ? prm->mask->dev : nullptr;
@@ -813,6 +824,14 @@ int gpv_solve_batch(gpv_context *ctx, const gpv_image *f, const gpv_image *g, co
         GPV_CUDA_TRY(cudaMemcpyAsync(prm->history, hist_dev, hist_bytes, cudaMemcpyDeviceToHost, ctx->stream));
     }
     GPV_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    // subsets that no launch took
+    for (int64_t i = n - invalid; i < n; i++) {
+        gpv_subset_result &o = out[order[i]];
+        std::memset(&o, 0, sizeof o);
+        std::memcpy(o.p, desc[order[i]].p0, sizeof o.p);
+        o.c_znssd = 4.0;
+        o.status = GPV_INVALID_SUBSET;
+    }
     return GPV_SUCCESS;
 }
 

@@ -907,7 +907,7 @@ int solve_launch(gpv_context *ctx, const SolveLaunch &L, cudaStream_t s) {
             A.g64 = nullptr;
         }
         if (!(prm->flags & GPV_SOLVE_RIGID_TEXTURE)) {
-            if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (96 + (size_t)L.n))) return rc;
+            if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (kTileWs + (size_t)L.n))) return rc;
             return tile_launch(ctx, A, L.n, SolveForm::kFagn, s);
         }
         int per_sm = 0;
@@ -927,7 +927,7 @@ int solve_launch(gpv_context *ctx, const SolveLaunch &L, cudaStream_t s) {
     }
     const bool runs64 = fp64 && !(prm->flags & GPV_SOLVE_RIGID_TEXTURE);
     if (runs64 || (!fp64 && !use_warp_kernel())) {
-        if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (96 + (size_t)L.n))) return rc;
+        if (int rc = ctx->tile_ws.ensure(sizeof(int32_t) * (kTileWs + (size_t)L.n))) return rc;
         return tile_launch(ctx, A, L.n, runs64 ? SolveForm::kFp64 : SolveForm::kMixed, s);
     }
     int workers, threads;

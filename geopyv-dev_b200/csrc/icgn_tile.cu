@@ -1222,7 +1222,7 @@ bool use_run_kernel();
 // Threads per block of the tiled kernel for subsets of radius r: the
 // autotuned choice when one was recorded for this radius class, else a
 // size rule (GPV_TILE_THREADS overrides).
-int tile_threads_for(gpv_context *ctx, int max_radius);
+int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n);
 
 // Raise a kernel's dynamic shared-memory limit to everything the device
 // allows beside its static shared memory, once per (device, kernel).  The
@@ -1298,12 +1298,14 @@ int query_nsmid(int *out) {
 int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cudaStream_t s) {
     const bool mixed = form == SolveForm::kMixed, fagn = form == SolveForm::kFagn;
     int32_t *ws = static_cast<int32_t *>(ctx->tile_ws.ptr);
-    int32_t *cnt = ws, *fill = ws + 16, *seg = ws + 32, *queues = ws + 64, *order_out = ws + 96;
-    GPV_CUDA_TRY(cudaMemsetAsync(ws, 0, 96 * sizeof(int32_t), s));
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    count_orders<<<blocks, 256, 0, s>>>(K.desc, K.order, (int)n, K.max_radius, cnt);
-    scatter_orders<<<blocks, 256, 0, s>>>(K.desc, K.order, (int)n, K.max_radius, cnt, fill, order_out, seg, K.out);
-    GPV_CUDA_TRY(cudaGetLastError());
+    int32_t *cnt = ws, *fill = ws + 16, *seg = ws + kTileWsSeg, *queues = ws + kTileWsQueue, *order_out = ws + kTileWs;
+    if (!ctx->seg_count_valid) {  // a host batch brings its partition with it
+        GPV_CUDA_TRY(cudaMemsetAsync(ws, 0, kTileWs * sizeof(int32_t), s));
+        const unsigned blocks = (unsigned)((n + 255) / 256);
+        count_orders<<<blocks, 256, 0, s>>>(K.desc, K.order, (int)n, K.max_radius, cnt);
+        scatter_orders<<<blocks, 256, 0, s>>>(K.desc, K.order, (int)n, K.max_radius, cnt, fill, order_out, seg, K.out);
+        GPV_CUDA_TRY(cudaGetLastError());
+    }
     struct Plan {
         int rmax = 0, nt = 0, layout = 0, cap = 0, blocks = 0, per_sm = 0;
         bool ps = false, rigid = false;  // one block per subset; rigid-texture template
@@ -1347,7 +1349,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             region = std::max(region, P.blocks * P.stride);
             continue;
         }
-        P.nt = tile_threads_for(ctx, P.rmax);
+        P.nt = tile_threads_for(ctx, P.rmax, n);
         P.layout = tile_layout_for(ctx, P.rmax);
         // persistent deformable segments run the run-layout kernel unless
         // GPV_SOLVE_KERNEL=tile asks for the tiled one
@@ -1397,8 +1399,10 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             P.blocks = (int)ctx->seg_count[q];
             slots = (int64_t)per_sm * ctx->n_smid;
         } else {
-            P.blocks = per_sm * ctx->num_sms;
-            slots = P.blocks;
+            // (no more blocks than subsets: an idle one costs its launch)
+            const int64_t nseg = ctx->seg_count_valid ? ctx->seg_count[q] : n;
+            P.blocks = (int)std::min<int64_t>(per_sm * ctx->num_sms, nseg);
+            slots = (int64_t)per_sm * ctx->num_sms;
         }
         region = std::max(region, slots * P.stride);
     }
@@ -1475,12 +1479,18 @@ bool use_run_kernel() {
     return !(v && v[0] == 't');
 }
 
-int tile_threads_for(gpv_context *ctx, int max_radius) {
+int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n) {
     if (ctx->force_threads) return ctx->force_threads;
     if (const char *v = getenv("GPV_TILE_THREADS")) {
         const int t = atoi(v);
         return t == 256 ? 256 : (t == 64 ? 64 : 128);
     }
+    // A batch that leaves every SM one subset at most is bound by one subset's
+    // latency: 256 threads (first order, radius 25: 91 against 94 us for 256
+    // subsets by the device call, a mesh's batches of tens 8 % shorter).  From
+    // two subsets per SM on, 128 threads share the SM better (576 subsets: 96
+    // against 110 us).
+    if (n <= ctx->num_sms) return 256;
     const int cls = max_radius <= 20 ? 0 : (max_radius <= 40 ? 1 : 2);
     if (ctx->tuned_threads[cls]) return ctx->tuned_threads[cls];
     return max_radius > 40 ? 256 : 128;

@@ -84,10 +84,9 @@ struct gpv_context {
     gpv::DevBuf queue;     // work-queue counters
     gpv::DevBuf desc_dev;  // staging for the host API
     gpv::DevBuf out_dev;
-    gpv::DevBuf order_dev;
     gpv::DevBuf hist_dev;
     gpv::DevBuf eval_dev;
-    gpv::DevBuf tile_ws;               // order partition + per-kernel queues
+    gpv::DevBuf tile_ws;               // order partition + per-kernel queues (kTileWs ints), work order
     cudaStream_t aux[2] = {nullptr, nullptr};  // extra streams for the per-order kernels
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     int mixed_blocks_per_sm = 0;
@@ -186,16 +185,20 @@ int mesh_drive(const double *nodes, int64_t n_nodes, const int64_t *elements, in
                gpv_subset_result *out, int32_t *rounds, gpv_mesh_stats *stats);
 // Colour ingest (load_grayscale + gaussian_blur_5x5): RGB8 (h, w, 3) -> u8 grey.
 int ingest_launch(const uint8_t *rgb_dev, int64_t h, int64_t w, uint8_t *grey_dev, cudaStream_t s);
-// Threads per block / template layout (0 compact, 1 padded rows, 2 tiles) of
-// the tiled solve for subsets up to max_radius: GPV_TILE_THREADS /
-// GPV_TILE_LAYOUT, else a candidate being timed, else the tuned choice.
-int tile_threads_for(gpv_context *ctx, int max_radius);
+// Threads per block (batches of n subsets) / template layout (0 compact, 1
+// padded rows, 2 tiles) of the tiled solve for subsets up to max_radius:
+// GPV_TILE_THREADS / GPV_TILE_LAYOUT, else a candidate being timed, else the
+// tuned choice.
+int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n);
 int tile_layout_for(gpv_context *ctx, int max_radius);
 // The (order, radius class) segment of the tiled solve that holds a valid
 // subset of radius r and warp order o (0 <= q < kTileSegs); a host batch's
 // per-segment counts let the launcher skip empty segments and size
 // one-block-per-subset grids.
 constexpr int kTileSegs = 12;
+// tile_ws: counts, fills, segments {start, count} (kTileWsSeg), work queues
+// (kTileWsQueue), then from kTileWs the work order by segment
+constexpr int kTileWs = 96, kTileWsSeg = 32, kTileWsQueue = 64;
 int tile_segment_of(int r, int o);
 // Number of SM identifiers (%nsmid) of the current device.
 int query_nsmid(int *out);
