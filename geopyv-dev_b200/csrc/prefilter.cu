@@ -9,18 +9,33 @@
 // That is a circular convolution with the periodised inverse filter
 //     h_N[m] = (1/N) sum_j cos(2 pi j m / N) / K(2 pi j / N),
 //     K(w)   = 11/20 + (13/30) cos w + (1/60) cos 2w,
-// whose spectrum is evaluated here in closed form once per line length N
-// (the kernel's FFT in the reference).  |h_N[m]| decays as 0.4306^|m|, so
-// |m| <= 44 reproduces the FFT result to FP64 rounding (1e-14 relative; see
-// tests/test_prefilter_*).  An image whose coefficients are kept in FP32
-// only uses |m| <= 28: the dropped taps sum to 2.7e-10 of the largest input
-// per pass, below FP32 rounding.  Both passes run in one kernel
-// (prefilter_fused): every thread slides a (2 MT + 1)-tap FP64 window along
-// 16 outputs of one line (taps are kernel parameters, i.e. constant-bank
-// operands), first along staged pixel rows, then down a ring of FP64
-// row-pass lines held in shared memory; the coefficients come out as FP32
-// (and optionally FP64), (h + 2b, w + 2b).  Images with a line shorter than
-// 89 samples take two simple kernels through an FP64 row-pass buffer.
+// whose poles are z_i and 1/z_i with z_i + 1/z_i = w_i = -13 +- sqrt(105)
+// (K = (w - w_1)(w - w_2) / 120 in w = z + 1/z), so by partial fractions
+//     h[m] = A_1 z_1^|m| + A_2 z_2^|m|,  z_1 = -0.4306, z_2 = -0.0431,
+// the sum of two decaying exponentials to either side: four first-order
+// recursions (M. Unser, A. Aldroubi, M. Eden, "B-spline signal processing",
+// IEEE Trans. Signal Process. 41, 1993, run them over whole lines; here they run
+// over blocks with a lead-in).  A thread makes kQ outputs of one line: the
+// recursions that come from the left start MT samples before them, those from
+// the right MT samples after, so the taps dropped are those past |m| = MT of a
+// direct filter: MT = 44 reproduces the FFT result to FP64 rounding (1e-14
+// relative; see tests/test_prefilter_*), and an image whose coefficients are
+// kept in FP32 only takes MT = 28 (dropped taps sum to 2.7e-10 of the largest
+// input per pass, below FP32 rounding).  That is 12 FP64 multiply-adds per
+// output and pass (MT = 28) against 57 of the direct filter this replaced,
+// whose bound was the FP64 pipe (55 % of its peak); now the pixel loads' latency
+// and the shared-memory reads bound it (FP64 pipe 17-25 %), so a warp has the
+// loads of kAhead lines in flight and three blocks share an SM (80 registers).
+// 4096^2 u16 207 -> 119 us, 2048^2 u8 63 -> 35, 911 x 1237 f64 with FP64
+// coefficients 102 -> 26, 4096^2 f32 with FP64 coefficients 596 -> 279.  Groups of kQ outputs start at multiples of kQ
+// of the padded line, so an output does not depend on how the rows are cut
+// into launches and blocks.  Both passes run in one kernel (prefilter_fused):
+// first along staged pixel rows, then down a ring of FP64 row-pass lines held in
+// shared memory; the coefficients come out as FP32 (and optionally FP64),
+// (h + 2b, w + 2b).  Images with a line shorter than 89 samples take every tap
+// of the periodised filter, whose spectrum is evaluated in closed form once per
+// line length N (the kernel's FFT in the reference), in two simple kernels
+// through an FP64 row-pass buffer.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -30,7 +45,7 @@
 namespace gpv {
 
 namespace {
-constexpr int kM = 44;             // taps on each side of the centre (FP64 coefficients)
+constexpr int kM = 44;             // lead-in of the recursions (FP64 coefficients)
 constexpr int kM32 = 28;           // the same when the coefficients are kept in FP32 only
 constexpr int kT = 2 * kM + 1;     // 89
 constexpr int kGroups = 8;         // warps per block
@@ -43,9 +58,50 @@ struct TapArg {
 std::mutex g_taps_mu;
 std::map<int64_t, Taps> g_taps;
 
-template <typename P>
-__device__ __forceinline__ double px_load(const P *p, int64_t i) {
-    return (double)p[i];
+// The two exponentials: poles z, weights A, and B = A z for the side that
+// starts one sample off the centre.
+struct Poles {
+    double z1, z2, a1, a2, b1, b2;
+};
+
+Poles poles() {
+    const double w1 = -13.0 + std::sqrt(105.0), w2 = -13.0 - std::sqrt(105.0);
+    Poles p;
+    p.z1 = 2.0 / (w1 - std::sqrt(w1 * w1 - 4.0));
+    p.z2 = 2.0 / (w2 - std::sqrt(w2 * w2 - 4.0));
+    const double g = 120.0 / (w1 - w2);
+    p.a1 = -g * p.z1 / (1.0 - p.z1 * p.z1);
+    p.a2 = g * p.z2 / (1.0 - p.z2 * p.z2);
+    p.b1 = p.a1 * p.z1;
+    p.b2 = p.a2 * p.z2;
+    return p;
+}
+
+// kQ outputs of a line from its 2 MT + kQ samples x(0 ..), output q at sample
+// MT + q.  Both sides advance together (four independent chains); the fast
+// pole needs W2 samples of lead-in only (0.0431^8 = 1.2e-11, ^13 = 1.8e-18).
+template <int MT, class X>
+__device__ __forceinline__ void exponentials(X x, const Poles &c, double (&acc)[kQ]) {
+    constexpr int W2 = MT <= 28 ? 8 : 13;
+    double p1 = 0.0, p2 = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int k = 0; k < MT + kQ; k++) {
+        {
+            const double v = x(k);
+            p1 = fma(c.z1, p1, v);
+            if (k >= MT - W2) p2 = fma(c.z2, p2, v);
+            const int q = k - MT;
+            if (q >= 0) acc[q] = fma(c.a1, p1, 2 * q < kQ - 1 ? c.a2 * p2 : fma(c.a2, p2, acc[q]));
+        }
+        const int sx = 2 * MT + kQ - 1 - k;
+        if (sx > MT) {
+            const double v = x(sx);
+            s1 = fma(c.z1, s1, v);
+            if (sx <= MT + kQ + W2) s2 = fma(c.z2, s2, v);
+            const int q = sx - 1 - MT;
+            if (q < kQ) acc[q] = fma(c.b1, s1, 2 * q < kQ - 1 ? fma(c.b2, s2, acc[q]) : c.b2 * s2);
+        }
+    }
 }
 
 // Both passes in one kernel.  A block owns a strip of kStrip padded columns
@@ -55,15 +111,13 @@ __device__ __forceinline__ double px_load(const P *p, int64_t i) {
 // FP64 lines that also holds the 2 MT lines before them, and the column pass
 // of kStep outputs reads that ring.  The FP64 row-pass lines never leave the
 // SM: DRAM sees the pixels (read once per strip; the halo columns of
-// neighbouring strips come from L2) and the coefficients written.  Each
-// output is the same FMA sequence, in the same order, as a separate row
-// pass and column pass would give (taps k = 0 .. 2 MT, increasing).
-//   row pass:    R[r][j] = sum_k tr[k] X[r][(j - MT + k) mod cw],
-//                X[r][jj] = px[r][clamp(jj - border, 0, w - 1)]
-//   column pass: C[i][j] = sum_k tc[k] R[clamp((i - MT + k) mod ch - border, 0, h - 1)][j]
+// neighbouring strips come from L2) and the coefficients written.
+//   row pass:    R[r] = the filter along X[r], X[r][jj] = px[r][clamp(jj mod cw - border, 0, w - 1)]
+//   column pass: C[.][j] = the filter down R[clamp(i mod ch - border, 0, h - 1)][j]
 constexpr int kStrip = 32;   // columns per block (one per lane in the column pass)
 constexpr int kStep = 128;   // output rows per step (8 warps x kQ)
 constexpr int kFusedThreads = kGroups * 32;
+constexpr int kAhead = 4;    // pixel lines a warp has in flight while staging
 static_assert(kStep == kGroups * kQ && kStrip == 2 * kQ, "one row-pass line per two threads, one output column per lane");
 
 // Staged pixel line pitch (elements) for kPxW pixels: lanes of a warp read 32
@@ -76,7 +130,7 @@ __host__ __device__ constexpr int px_pitch() {
 
 template <typename P, int MT>
 struct Fused {
-    static constexpr int kTaps = 2 * MT + 1, kHalo = 2 * MT;
+    static constexpr int kHalo = 2 * MT;
     static constexpr int kRing = kStep + kHalo;   // FP64 row-pass lines held
     static constexpr int kRingPitch = kStrip + 1;  // doubles
     static constexpr int kPxW = kStrip + kHalo;   // pixels per staged line
@@ -86,9 +140,9 @@ struct Fused {
 };
 
 template <typename P, int MT>
-__global__ void __launch_bounds__(kFusedThreads) prefilter_fused(const P *__restrict__ px, int64_t h, int64_t w,
+__global__ void __launch_bounds__(kFusedThreads, 3) prefilter_fused(const P *__restrict__ px, int64_t h, int64_t w,
                                                                 int64_t border, int64_t cw, int64_t ch, int64_t i_lo,
-                                                                int64_t i_hi, int64_t seg, TapArg tr, TapArg tc,
+                                                                int64_t i_hi, int64_t seg, Poles poles,
                                                                 float *__restrict__ c32, int64_t pitch32,
                                                                 double *__restrict__ c64, int64_t pitch64) {
     using G = Fused<P, MT>;
@@ -96,7 +150,7 @@ __global__ void __launch_bounds__(kFusedThreads) prefilter_fused(const P *__rest
     double *ring = smem;
     P *pxs = reinterpret_cast<P *>(reinterpret_cast<unsigned char *>(smem) + G::kRingBytes);
     const int64_t j0 = (int64_t)blockIdx.x * kStrip;
-    const int64_t i_beg = i_lo + (int64_t)blockIdx.y * seg;
+    const int64_t i_beg = i_lo + (int64_t)blockIdx.y * seg;  // a multiple of kQ, as i_lo and seg are
     const int64_t i_end = i_beg + seg < i_hi ? i_beg + seg : i_hi;
     if (i_beg >= i_end) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -118,33 +172,38 @@ __global__ void __launch_bounds__(kFusedThreads) prefilter_fused(const P *__rest
     auto produce = [&](int64_t row0, int n, int dst) {
         int base = (int)(row0 % ch);  // row0 >= -MT
         if (base < 0) base += (int)ch;
-        for (int rr = wid; rr < n; rr += kGroups) {
-            int ii = base + rr;
-            while (ii >= (int)ch) ii -= (int)ch;
-            int r = ii - (int)border;
-            r = r < 0 ? 0 : (r > (int)h - 1 ? (int)h - 1 : r);
-            const P *src = px + (int64_t)r * w;
-            P *d = pxs + rr * G::kPxPitch + lane;
+        // kAhead lines of a warp at a time, their loads together in flight
+#pragma unroll 1
+        for (int r0 = wid; r0 < n; r0 += kAhead * kGroups) {
+            P v[kAhead][kCols];
 #pragma unroll
-            for (int m = 0; m < kCols; m++)
-                if (csrc[m] >= 0) d[32 * m] = src[csrc[m]];
+            for (int a = 0; a < kAhead; a++) {
+                const int rr = r0 + a * kGroups;
+                int ii = base + min(rr, n - 1);
+                while (ii >= (int)ch) ii -= (int)ch;
+                const int r = min(max(ii - (int)border, 0), (int)h - 1);
+                const P *src = px + (int64_t)r * w;
+#pragma unroll
+                for (int m = 0; m < kCols; m++)
+                    if (csrc[m] >= 0) v[a][m] = src[csrc[m]];
+            }
+#pragma unroll
+            for (int a = 0; a < kAhead; a++) {
+                const int rr = r0 + a * kGroups;
+                if (rr < n) {
+                    P *d = pxs + rr * G::kPxPitch + lane;
+#pragma unroll
+                    for (int m = 0; m < kCols; m++)
+                        if (csrc[m] >= 0) d[32 * m] = v[a][m];
+                }
+            }
         }
         __syncthreads();
         const int rr = (wid & 3) * 32 + lane, half = wid >> 2;
         if (rr < n) {
             const P *x = pxs + rr * G::kPxPitch + half * kQ;
             double acc[kQ];
-#pragma unroll
-            for (int q = 0; q < kQ; q++) acc[q] = 0.0;
-#pragma unroll
-            for (int sx = 0; sx < kQ + G::kHalo; sx++) {
-                const double xv = (double)x[sx];
-#pragma unroll
-                for (int q = 0; q < kQ; q++) {
-                    const int k = sx - q;
-                    if (k >= 0 && k < G::kTaps) acc[q] = fma(tr.h[k], xv, acc[q]);
-                }
-            }
+            exponentials<MT>([&](int sx) { return (double)x[sx]; }, poles, acc);
             double *o = ring + (dst + rr) * G::kRingPitch + half * kQ;
 #pragma unroll
             for (int q = 0; q < kQ; q++) o[q] = acc[q];
@@ -156,22 +215,13 @@ __global__ void __launch_bounds__(kFusedThreads) prefilter_fused(const P *__rest
     produce(i_beg - MT, G::kHalo, 0);
     for (int64_t done = 0; done < i_end - i_beg; done += kStep) {
         const int n = (int)(i_end - i_beg - done < kStep ? i_end - i_beg - done : kStep);
-        produce(i_beg + MT + done, n, G::kHalo);
+        // whole groups of lines: the last group's recursions start past the segment's end
+        produce(i_beg + MT + done, (n + kQ - 1) / kQ * kQ, G::kHalo);
         // column pass: lane = column, warp wid = outputs [wid kQ, wid kQ + kQ) of this step
         if (wid * kQ < n) {
             const double *x = ring + (wid * kQ) * G::kRingPitch + lane;
             double acc[kQ];
-#pragma unroll
-            for (int q = 0; q < kQ; q++) acc[q] = 0.0;
-#pragma unroll
-            for (int sx = 0; sx < kQ + G::kHalo; sx++) {
-                const double xv = x[sx * G::kRingPitch];
-#pragma unroll
-                for (int q = 0; q < kQ; q++) {
-                    const int k = sx - q;
-                    if (k >= 0 && k < G::kTaps) acc[q] = fma(tc.h[k], xv, acc[q]);
-                }
-            }
+            exponentials<MT>([&](int sx) { return x[sx * G::kRingPitch]; }, poles, acc);
             const int64_t j = j0 + lane;
             if (j < cw) {
 #pragma unroll
@@ -237,11 +287,6 @@ void fill_taparg(const Taps &t, TapArg &a) {
     for (int k = 0; k < nt; k++) a.h[k] = t.h[t.mr - k + t.ml];
 }
 
-// The central 2 mt + 1 taps of a long line's filter (|m| <= mt), reversed.
-void fill_taparg_central(const Taps &t, int mt, TapArg &a) {
-    for (int k = 0; k <= 2 * mt; k++) a.h[k] = t.h[t.ml + mt - k];
-}
-
 // Blocks per SM of one fused instantiation at its shared memory (cached per
 // device); also raises the kernel's dynamic shared-memory limit.
 template <typename P, int MT>
@@ -264,45 +309,51 @@ int fused_blocks_per_sm(int *bps) {
 }
 
 // Coefficient rows [lo, hi) of an image whose lines both have at least kT
-// samples, MT taps on each side.  Segments of rows split the work into about
-// three waves of blocks, each segment at least 6 x 2 MT rows long (its 2 MT
-// lead-in row-pass lines are the only work done twice).
+// samples, lead-in MT; lo is a multiple of kQ, and hi too unless it is the last
+// row's end (the groups of outputs are cut at multiples of kQ).  The rows are
+// split into the number of segments that makes the last wave of blocks end
+// first, each segment paying for its 2 MT lead-in lines: a 4096^2 image has
+// blocks for several waves whatever the split, but a strip per 32 columns
+// of a 1237-pixel-wide one leaves three quarters of the SMs idle unless its
+// rows are cut short.
 template <typename P, int MT>
-int launch_fused(gpv_image *img, const P *px, const Taps &tr, const Taps &tc, cudaStream_t s, int64_t lo, int64_t hi) {
+int launch_fused(gpv_image *img, const P *px, cudaStream_t s, int64_t lo, int64_t hi) {
     if (hi <= lo) return GPV_SUCCESS;
     int bps = 1;
     if (int rc = fused_blocks_per_sm<P, MT>(&bps)) return rc;
-    TapArg ar, ac;
-    fill_taparg_central(tr, MT, ar);
-    fill_taparg_central(tc, MT, ac);
     const int64_t strips = (img->cw + kStrip - 1) / kStrip, rows = hi - lo;
-    const int64_t target = 3LL * bps * std::max(1, img->ctx->num_sms);
-    int64_t segs = std::max<int64_t>(1, (target + strips - 1) / strips);
-    segs = std::min<int64_t>(segs, std::max<int64_t>(1, rows / (6 * 2 * MT)));
-    const int64_t seg = (rows + segs - 1) / segs;
-    segs = (rows + seg - 1) / seg;
+    const int64_t slots = (int64_t)bps * std::max(1, img->ctx->num_sms);
+    int64_t seg = rows, best = INT64_MAX;
+    for (int64_t n = 1; n <= (rows + kQ - 1) / kQ; n++) {
+        const int64_t len = ((rows + n - 1) / n + kQ - 1) / kQ * kQ, k = (rows + len - 1) / len;
+        const int64_t cost = (strips * k + slots - 1) / slots * (len + 2 * MT);
+        if (cost < best) {
+            best = cost;
+            seg = len;
+        }
+    }
+    const int64_t segs = (rows + seg - 1) / seg;
+    static const Poles kPoles = poles();
     prefilter_fused<P, MT><<<dim3((unsigned)strips, (unsigned)segs), kFusedThreads, Fused<P, MT>::kSmem, s>>>(
-        px, img->h, img->w, img->border, img->cw, img->ch, lo, hi, seg, ar, ac, img->c32, img->pitch32, img->c64,
+        px, img->h, img->w, img->border, img->cw, img->ch, lo, hi, seg, kPoles, img->c32, img->pitch32, img->c64,
         img->pitch64);
     GPV_CUDA_TRY(cudaGetLastError());
     return GPV_SUCCESS;
 }
 
 template <typename P>
-int launch_fused_rows(gpv_image *img, const P *px, const Taps &tr, const Taps &tc, cudaStream_t s, int64_t lo,
-                      int64_t hi) {
+int launch_fused_rows(gpv_image *img, const P *px, cudaStream_t s, int64_t lo, int64_t hi) {
     // coefficients kept in FP32 only: |m| <= kM32
-    return img->c64 == nullptr ? launch_fused<P, kM32>(img, px, tr, tc, s, lo, hi)
-                               : launch_fused<P, kM>(img, px, tr, tc, s, lo, hi);
+    return img->c64 == nullptr ? launch_fused<P, kM32>(img, px, s, lo, hi) : launch_fused<P, kM>(img, px, s, lo, hi);
 }
 
 bool long_lines(const gpv_image *img) { return img->cw >= kT && img->ch >= kT; }
 
 template <typename P>
 int run_prefilter(gpv_image *img, const P *px, cudaStream_t s) {
+    if (long_lines(img)) return launch_fused_rows(img, px, s, 0, img->ch);
     const Taps &tr = taps_for(img->cw);
     const Taps &tc = taps_for(img->ch);
-    if (long_lines(img)) return launch_fused_rows(img, px, tr, tc, s, 0, img->ch);
     // a short line: every circulant tap, through the FP64 row-pass buffer
     {
         const int nt = tr.ml + tr.mr + 1;
@@ -367,17 +418,15 @@ const Taps &taps_for(int64_t n) {
 
 namespace {
 // Host pixels in row chunks into img->px_dev on the copy stream cs.  As each
-// chunk lands, the coefficient rows whose lines all come from rows already
-// landed are filtered on s, so the copies overlap the filtering; the first
-// MT coefficient rows (their column taps wrap to the image's last rows) go
-// after the last chunk.  Images with a short line take the whole copy, then
+// chunk lands, the groups of coefficient rows whose lines all come from rows
+// already landed are filtered on s, so the copies overlap the filtering; the
+// first groups (their lines wrap to the image's last rows) go after the last
+// chunk.  Images with a short line take the whole copy, then
 // the ordinary prefilter.
 template <typename P>
 int prefilter_host(gpv_image *img, const P *px_host, cudaStream_t s, cudaStream_t cs, cudaEvent_t *ev, int nev) {
     P *dst = static_cast<P *>(img->px_dev);
     const size_t row_bytes = sizeof(P) * (size_t)img->w;
-    const Taps &tr = taps_for(img->cw);
-    const Taps &tc = taps_for(img->ch);
     // rows per copy: ceil(h / (nev - 1)) rounded up to 32, so at most nev - 1
     // chunks (events ev[1 .. nev-1]) cover the image
     const int64_t chunk = ((img->h + nev - 2) / (nev - 1) + 31) / 32 * 32;
@@ -391,7 +440,9 @@ int prefilter_host(gpv_image *img, const P *px_host, cudaStream_t s, cudaStream_
         return run_prefilter(img, static_cast<const P *>(dst), s);
     }
     const int64_t mt = img->c64 == nullptr ? kM32 : kM;
-    int64_t lo = mt;  // coefficient rows [0, mt) wait for the last chunk
+    // coefficient rows [0, first) wait for the last chunk (their lines wrap to the last rows)
+    const int64_t first = (mt + kQ - 1) / kQ * kQ;
+    int64_t lo = first;
     int k = 1;
     for (int64_t r0 = 0; r0 < img->h; r0 += chunk, k++) {
         // the last event takes whatever rows remain (never an event past ev[nev - 1])
@@ -400,15 +451,15 @@ int prefilter_host(gpv_image *img, const P *px_host, cudaStream_t s, cudaStream_
                                      cudaMemcpyHostToDevice, cs));
         GPV_CUDA_TRY(cudaEventRecord(ev[k], cs));
         GPV_CUDA_TRY(cudaStreamWaitEvent(s, ev[k], 0));
-        // coefficient row i reads image rows up to min(h - 1, i + mt - border)
+        // a group of coefficient rows ending at i reads image rows below min(h, i + mt - border)
         const int64_t landed = r0 + nr;
-        const int64_t hi = landed >= img->h ? img->ch : std::min(img->ch, landed - mt + img->border);
+        const int64_t hi = landed >= img->h ? img->ch : (landed - mt + img->border) / kQ * kQ;
         if (hi > lo) {
-            if (int rc = launch_fused_rows(img, static_cast<const P *>(dst), tr, tc, s, lo, hi)) return rc;
+            if (int rc = launch_fused_rows(img, static_cast<const P *>(dst), s, lo, hi)) return rc;
             lo = hi;
         }
     }
-    return launch_fused_rows(img, static_cast<const P *>(dst), tr, tc, s, 0, mt);
+    return launch_fused_rows(img, static_cast<const P *>(dst), s, 0, first);
 }
 }  // namespace
 

@@ -134,3 +134,20 @@ def test_pinned_chunked_update_equals_pageable_update(gpv_mod, dtype, keep_f64, 
     ga, gb = a.grain(maps=True), b.grain(maps=True)
     assert ga["correlation_length"] == gb["correlation_length"]
     assert np.array_equal(ga["maps"], gb["maps"])
+
+
+@pytest.mark.parametrize("keep_f64", [False, True])
+@pytest.mark.parametrize("shape", [(49, 49), (50, 89), (57, 1000), (105, 64), (119, 121), (345, 51), (700, 49)])
+def test_group_and_strip_edges_match_oracle(oracle, gpv_mod, shape, keep_f64):
+    """Padded lines of 89 samples (the shortest the recursions take), one more or
+    one less than whole groups of 16 outputs and strips of 32 columns, and one
+    strip cut into many segments of rows: the oracle's coefficients within
+    1e-8 (FP64) and 2e-7 (FP32) of the largest, pinned (chunked) or not."""
+    rng = np.random.default_rng(shape[0] + 3 * shape[1])
+    img = rng.integers(0, 256, shape).astype(np.uint8)
+    ref = oracle.get_c(img.astype(np.float64), 20)
+    im = gpv_mod.Image(image_gs=img, border=20, keep_f64=keep_f64)
+    scale = np.abs(ref).max()
+    assert np.abs(im.coef().astype(np.float64) - ref).max() <= 2e-7 * scale
+    if keep_f64:
+        assert np.abs(im.coef(f64=True) - ref).max() <= 1e-8 * scale
