@@ -35,7 +35,7 @@
 //    pivoting while the pivots stay near 1, else with pivoting.
 // Measured against one sweep-per-sum block of 256 threads with taps through L1
 // (icgn_fp64, fagn_kernel; 254 registers, 8 warps per SM, FP64 pipe 14 % and
-// 29 % busy): 8,836 second-order subsets of radius 30 12.53 -> 2.68 ms (FP64
+// 29 % busy): 8,836 second-order subsets of radius 30 12.53 -> 2.40 ms (FP64
 // pipe 40 %), 2,401 first-order FAGN solves of radius 25 on FP32 coefficients
 // 1.27 -> 0.62 ms (47 %).
 // Samples that can meet the image's edge, and windows that do not fit in
@@ -128,6 +128,18 @@ __device__ __forceinline__ double dot6(const double (&c)[6], const double (&b)[6
     return fma(c[4], b[4], fma(c[2], b[2], c[0] * b[0])) + fma(c[5], b[5], fma(c[3], b[3], c[1] * b[1]));
 }
 
+// A record's parts, read once per sweep: not kept in L1.
+__device__ __forceinline__ double2 ld_pair(const double2 *p) {
+    double2 v;
+    asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_one(const double *p) {
+    double v;
+    asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 // Gauss-Jordan inverse with partial pivoting by one thread, for matrices that
 // the Cholesky factor rejects; false when no pivot is left.
 template <int M>
@@ -170,7 +182,7 @@ __device__ __noinline__ bool compose2_any(const double *p, const double *d, doub
 // One solve.  scratch (doubles, nslot slots per array, slot j * T + t for
 // pixel j of run t): the gradient pair, f - s (s the subset's level), g; for
 // FAGN the target's gradient pair too; then one word of pixel bits per run.
-template <int ORDER, int NT, bool FAGN, typename C>
+template <int ORDER, int NT, bool FAGN, typename C, bool ETA>
 __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, double *base, double *win,
                              Smem64<NT / 32> &sm) {
     const KArgs &A = R.k;
@@ -473,7 +485,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             const double Ax = fma(fma(uxx, dxf, ux), dxf, ox), Ay = fma(fma(vxx, dxf, vx), dxf, oy);
             const double Bx = fma(uxy, dxf, uy), By = fma(vxy, dxf, vy);
             double m0x = 0.0, m0y = 0.0, m1x = 0.0, m1y = 0.0, m2x = 0.0, m2y = 0.0;
-            auto take = [&](int j, double dyf, double g, double hx, double hy) {
+            auto take = [&](int j, double dyf, double g, double hx, double hy, double2 gf, double fs) {
                 const int sl = j * T + t;
                 const bool in = (vm >> j) & 1u;
                 if constexpr (FAGN) {
@@ -483,8 +495,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     sb += b;
                     sbb = fma(b, b, sbb);
                 } else {
-                    const double2 gf = RG[sl];
-                    const double a = in ? RF[sl] - fms : 0.0, b = in ? g - cg : 0.0;
+                    const double a = in ? fs - fms : 0.0, b = in ? g - cg : 0.0;
                     const double e = fma(-rho, b, a);
                     sb += b;
                     sbb = fma(b, b, sbb);
@@ -505,6 +516,12 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
 #pragma unroll
                 for (int j = 0; j < kK; j++) {
                     const double dyf = dy0 + j;
+                    double2 gf = make_double2(0.0, 0.0);  // from L2: asked for at the sample's start
+                    double fs = 0.0;
+                    if constexpr (!FAGN) {
+                        gf = ld_pair(RG + j * T + t);
+                        fs = ld_one(RF + j * T + t);
+                    }
                     double Lx = Ax, Ly = Ay;
                     if (ORDER == 1) { Lx = fma(Bx, dyf, Lx); Ly = fma(By, dyf, Ly); }
                     if (ORDER == 2) { Lx = fma(fma(uyy, dyf, Bx), dyf, Lx); Ly = fma(fma(vyy, dyf, By), dyf, Ly); }
@@ -545,7 +562,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                         for (int rr = 0; rr < 6; rr++) sr[rr] = dot6(Rg[(j + rr) % 6], w);
                         hx = dot6(sr, aw);
                     }
-                    take(j, dyf, g, hx, hy);
+                    take(j, dyf, g, hx, hy, gf, fs);
                 }
             } else {
 #pragma unroll 1
@@ -568,7 +585,8 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                         if constexpr (FAGN) g = contract_grad<double>(q, cp, a, da, b, db, hx, hy);
                         else g = contract<double>(q, cp, a, b);
                     }
-                    take(j, dyf, g, hx, hy);
+                    if constexpr (FAGN) take(j, dyf, g, hx, hy, make_double2(0.0, 0.0), 0.0);
+                    else take(j, dyf, g, hx, hy, RG[j * T + t], RF[j * T + t]);
                 }
             }
             if constexpr (!FAGN) {
@@ -776,8 +794,8 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
 
     // ---- eta diagnostic at the last sampled warp (optional) -----------------
     double eu = 0.0, ev = 0.0;
-    const bool want_eta = (A.flags & GPV_SOLVE_ETA) && iters > 0 && status == GPV_OK;
-    if (want_eta) {
+    const bool want_eta = ETA && iters > 0 && status == GPV_OK;
+    if (ETA && want_eta) {
         const double *pp = sm.pprev;
         const double X0 = cx + pp[0], Y0 = cy + pp[1];
         const double bxd = floor(X0), byd = floor(Y0);
@@ -845,9 +863,12 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
     }
 }
 
-// Blocks take subsets of their segment from the queue.
-template <int ORDER, int NT, bool FAGN, typename C>
-__global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) icgn_runs64(RunArgs R) {
+// Blocks take subsets of their segment from the queue.  Three blocks of 128
+// threads per SM (168 registers); the second-order ICGN sweep, whose sums alone
+// take 70 registers, does better with two at 255 and no spills (2.40 against
+// 2.55 ms on 8,836 subsets of radius 30; first order 1.95 against 1.81).
+template <int ORDER, int NT, bool FAGN, typename C, bool ETA>
+__global__ void __launch_bounds__(NT, NT == 128 ? (ORDER == 2 && !FAGN ? 2 : 3) : 1) icgn_runs64(RunArgs R) {
     extern __shared__ double2 win2[];
     __shared__ Smem64<NT / 32> sm;
     const KArgs &A = R.k;
@@ -861,20 +882,21 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) icgn_runs64(RunArgs R) 
         if (item >= count) break;
         const int idx = A.order[start + item];
         const gpv_subset_desc d = A.desc[idx];
-        run64_subset<ORDER, NT, FAGN, C>(R, idx, d, base, reinterpret_cast<double *>(win2), sm);
+        run64_subset<ORDER, NT, FAGN, C, ETA>(R, idx, d, base, reinterpret_cast<double *>(win2), sm);
     }
 }
 
-template <int NT, bool FAGN, typename C>
+template <int NT, bool FAGN, typename C, bool ETA>
 const void *kernel64_t(int order) {
-    return order == 2 ? (const void *)icgn_runs64<2, NT, FAGN, C>
-                      : (order == 1 ? (const void *)icgn_runs64<1, NT, FAGN, C> : (const void *)icgn_runs64<0, NT, FAGN, C>);
+    return order == 2 ? (const void *)icgn_runs64<2, NT, FAGN, C, ETA>
+                      : (order == 1 ? (const void *)icgn_runs64<1, NT, FAGN, C, ETA>
+                                    : (const void *)icgn_runs64<0, NT, FAGN, C, ETA>);
 }
 
-template <int NT>
+template <int NT, bool ETA>
 const void *kernel64_nt(int order, bool fagn, bool c64) {
-    if (!fagn) return kernel64_t<NT, false, double>(order);
-    return c64 ? kernel64_t<NT, true, double>(order) : kernel64_t<NT, true, float>(order);
+    if (!fagn) return kernel64_t<NT, false, double, ETA>(order);
+    return c64 ? kernel64_t<NT, true, double, ETA>(order) : kernel64_t<NT, true, float, ETA>(order);
 }
 
 }  // namespace
@@ -893,8 +915,9 @@ int64_t run64_scratch_doubles(int nslot, bool fagn) {
     return (fagn ? 6 : 4) * (int64_t)nslot + nslot / (2 * kK) + 16;
 }
 
-const void *run64_kernel(int order, int nt, bool fagn, bool c64) {
-    return nt == 256 ? kernel64_nt<256>(order, fagn, c64) : kernel64_nt<128>(order, fagn, c64);
+const void *run64_kernel(int order, int nt, bool fagn, bool c64, bool eta) {
+    if (eta) return nt == 256 ? kernel64_nt<256, true>(order, fagn, c64) : kernel64_nt<128, true>(order, fagn, c64);
+    return nt == 256 ? kernel64_nt<256, false>(order, fagn, c64) : kernel64_nt<128, false>(order, fagn, c64);
 }
 
 int run64_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,

@@ -1336,7 +1336,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             // windows of three blocks fit), 256 threads where fewer windows fit
             P.nt = P.rmax > 32 ? 256 : 128;
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
-            P.fn = run64_kernel(order, P.nt, fagn, K.f64 != nullptr);
+            P.fn = run64_kernel(order, P.nt, fagn, K.f64 != nullptr, (K.flags & GPV_SOLVE_ETA) != 0);
             int max_bytes = 0;
             if (int rc = allow_max_dynamic_smem(P.fn, &max_bytes)) return rc;
             P.cap = std::min(run64_window_cap(P.rmax), max_bytes / (int)sizeof(double) / 4 * 4);

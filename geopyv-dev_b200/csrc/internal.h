@@ -214,7 +214,7 @@ int run_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem
 // icgn_runs64.cu: the FP64 solves (ICGN, FAGN) in run layout
 int run64_window_cap(int rmax);
 int64_t run64_scratch_doubles(int nslot, bool fagn);
-const void *run64_kernel(int order, int nt, bool fagn, bool c64);
+const void *run64_kernel(int order, int nt, bool fagn, bool c64, bool eta);
 int run64_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,
                  const int32_t *seg, int *queue, int win_cap, int nslot);
 int solve_noalloc_launch(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const gpv_subset_desc *desc_dev,
