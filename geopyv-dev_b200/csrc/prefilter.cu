@@ -21,12 +21,12 @@
 // direct filter: MT = 44 reproduces the FFT result to FP64 rounding (1e-14
 // relative; see tests/test_prefilter_*), and an image whose coefficients are
 // kept in FP32 only takes MT = 28 (dropped taps sum to 2.7e-10 of the largest
-// input per pass, below FP32 rounding).  That is 12 FP64 multiply-adds per
+// input per pass, below FP32 rounding).  That is 14 FP64 multiply-adds per
 // output and pass (MT = 28) against 57 of the direct filter this replaced,
 // whose bound was the FP64 pipe (55 % of its peak); now the pixel loads' latency
 // and the shared-memory reads bound it (FP64 pipe 17-25 %), so a warp has the
 // loads of kAhead lines in flight and three blocks share an SM (80 registers).
-// 4096^2 u16 207 -> 119 us, 2048^2 u8 63 -> 35, 911 x 1237 f64 with FP64
+// 4096^2 u16 207 -> 125 us, 2048^2 u8 63 -> 37, 911 x 1237 f64 with FP64
 // coefficients 102 -> 26, 4096^2 f32 with FP64 coefficients 596 -> 279.  Groups of kQ outputs start at multiples of kQ
 // of the padded line, so an output does not depend on how the rows are cut
 // into launches and blocks.  Both passes run in one kernel (prefilter_fused):
@@ -62,6 +62,7 @@ std::map<int64_t, Taps> g_taps;
 // starts one sample off the centre.
 struct Poles {
     double z1, z2, a1, a2, b1, b2;
+    double t1;  // A_1 z_1^(kM32 + 1): what a tap past |m| = kM32 weighs
 };
 
 Poles poles() {
@@ -74,32 +75,42 @@ Poles poles() {
     p.a2 = g * p.z2 / (1.0 - p.z2 * p.z2);
     p.b1 = p.a1 * p.z1;
     p.b2 = p.a2 * p.z2;
+    p.t1 = p.a1 * std::pow(p.z1, kM32 + 1);
     return p;
 }
 
 // kQ outputs of a line from its 2 MT + kQ samples x(0 ..), output q at sample
 // MT + q.  Both sides advance together (four independent chains); the fast
 // pole needs W2 samples of lead-in only (0.0431^8 = 1.2e-11, ^13 = 1.8e-18).
+// At MT = kM32 the slow pole's taps past |m| = MT, which the lead-in of the
+// other outputs brings with it, are taken off again (the chain's state MT + 1
+// samples back, times t1): every output is the filter of 2 MT + 1 taps, to FP64
+// rounding, wherever it lies in its group.
 template <int MT, class X>
 __device__ __forceinline__ void exponentials(X x, const Poles &c, double (&acc)[kQ]) {
+    constexpr bool kCut = MT == kM32;
     constexpr int W2 = MT <= 28 ? 8 : 13;
     double p1 = 0.0, p2 = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < kQ; q++) acc[q] = 0.0;
 #pragma unroll
     for (int k = 0; k < MT + kQ; k++) {
         {
             const double v = x(k);
             p1 = fma(c.z1, p1, v);
             if (k >= MT - W2) p2 = fma(c.z2, p2, v);
+            if (kCut && k + 1 < kQ) acc[k + 1] = fma(-c.t1, p1, acc[k + 1]);
             const int q = k - MT;
-            if (q >= 0) acc[q] = fma(c.a1, p1, 2 * q < kQ - 1 ? c.a2 * p2 : fma(c.a2, p2, acc[q]));
+            if (q >= 0) acc[q] = fma(c.a1, p1, fma(c.a2, p2, acc[q]));
         }
         const int sx = 2 * MT + kQ - 1 - k;
         if (sx > MT) {
             const double v = x(sx);
             s1 = fma(c.z1, s1, v);
             if (sx <= MT + kQ + W2) s2 = fma(c.z2, s2, v);
+            if (kCut && sx > 2 * MT) acc[sx - 2 * MT - 1] = fma(-c.t1, s1, acc[sx - 2 * MT - 1]);
             const int q = sx - 1 - MT;
-            if (q < kQ) acc[q] = fma(c.b1, s1, 2 * q < kQ - 1 ? fma(c.b2, s2, acc[q]) : c.b2 * s2);
+            if (q < kQ) acc[q] = fma(c.b1, s1, fma(c.b2, s2, acc[q]));
         }
     }
 }
