@@ -91,6 +91,30 @@ __device__ __forceinline__ bool mask_ok(const KArgs &A, int cxi, int cyi, int ox
     return A.mask[(int64_t)Y * A.mw + X] != 0;
 }
 
+// The three grain maps (fxx, fyy, fxy; rows x cols FP32) at (x = column,
+// y = row), bilinear, clamped (GrainMaps::sample, src/texture.rs:125-143).
+__device__ __forceinline__ void grain_sample(const float *maps, int rows, int cols, double x, double y, float h[3]) {
+    x = fmin(fmax(x, 0.0), (double)(cols - 1));
+    y = fmin(fmax(y, 0.0), (double)(rows - 1));
+    const int x0 = min((int)floor(x), max(cols - 2, 0)), y0 = min((int)floor(y), max(rows - 2, 0));
+    const int x1 = min(x0 + 1, cols - 1), y1 = min(y0 + 1, rows - 1);
+    const double tx = x - (double)x0, ty = y - (double)y0;
+    const int64_t np = (int64_t)rows * cols;
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+        const float *M = maps + m * np;
+        h[m] = (float)((1.0 - ty) * ((1.0 - tx) * M[(int64_t)y0 * cols + x0] + tx * M[(int64_t)y0 * cols + x1]) +
+                       ty * ((1.0 - tx) * M[(int64_t)y1 * cols + x0] + tx * M[(int64_t)y1 * cols + x1]));
+    }
+}
+
+// Green-Lagrange strain [Exx, Eyy, Exy] (src/texture.rs:200-206).
+__device__ __forceinline__ void green_lagrange(float ux, float vx, float uy, float vy, float &e0, float &e1, float &e2) {
+    e0 = ux + 0.5f * (ux * ux + vx * vx);
+    e1 = vy + 0.5f * (uy * uy + vy * vy);
+    e2 = 0.5f * (uy + vx) + 0.5f * (ux * uy + vx * vy);
+}
+
 // ---------------------------------------------------------------------
 // Warp composition (compose_icgn, src/subset.rs:487-611) in FP64.
 // Order 2 needs only rows 3 and 4 of W_old * W_delta^-1 (the u and v rows

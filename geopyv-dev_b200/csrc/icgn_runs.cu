@@ -49,6 +49,11 @@
 //    and the steepest-descent products) are FP32 over one run (at most K
 //    samples), then FP64 per thread and across the block in a fixed order
 //    (deterministic).
+//  * Rigid texture (RIGID; orders 1 and 2): the grain maps sampled per pixel at
+//    setup, and a template pass per iteration with the sums of its correction G
+//    (the run's four pixels' loads together in flight); the sample loop only adds
+//    G to its cross term.  14,420 second-order subsets of radius 30 4.33 ms in the
+//    tiled kernel, 3.2 here (deformable 2.0).
 // Subsets whose warped square leaves the image or the staged window take a
 // clamped per-sample path (the reference's edge clamp, src/image.rs:129-132),
 // reading the window with clamped indices or global memory.
@@ -203,6 +208,12 @@ __device__ __forceinline__ float4 ld_rec(const float4 *p) {
     return v;
 }
 
+__device__ __forceinline__ float ld_once(const float *p) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 // One coefficient row against the column weights: sum_k b_k c_k with the
 // pairs (c_k, c_{5-k}) x (b_k, b_{5-k}).
 __device__ __forceinline__ float row_dot(const float (&c)[6], const float2 B[3]) {
@@ -285,7 +296,7 @@ __device__ __forceinline__ void acc_expand(const RunAcc &a, float dxf, float2 (&
 template <int ORDER, int NT, int K>
 __device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, const float *__restrict__ g32, int64_t pitch32,
                                      int w, int h, int B, const int2 *tasks, int T, const float4 *REC, float *RSG,
-                                     const int *RVM, double cx, double cy, double fms, double dn, double df, double gm,
+                                     const int *RVM, const float *RTG, double cx, double cy, double fms, double dn, double df, double gm,
                                      double dg, double *eu, double *ev) {
     constexpr int M = Ord<ORDER>::M;
     const int tid = threadIdx.x;
@@ -333,7 +344,7 @@ __device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, 
                     }
                 }
                 const float4 rec = REC[sl];
-                fn((double)rec.z + fms, (double)rec.x, (double)rec.y, (double)RSG[sl] - gm, dx, dy);
+                fn((double)rec.z + (RTG ? (double)RTG[sl] : 0.0) + fms, (double)rec.x, (double)rec.y, (double)RSG[sl] - gm, dx, dy);
             }
         }
     };
@@ -344,7 +355,7 @@ __device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, 
     *ev = v;
 }
 
-template <int ORDER, int NT, int K, bool KAHAN, bool ETA>
+template <int ORDER, int NT, int K, bool KAHAN, bool ETA, bool RIGID>
 __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, float *base, float *win,
                            RunSmem<NT / 32> &sm) {
     const KArgs &A = R.k;
@@ -361,6 +372,10 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     float4 *REC = reinterpret_cast<float4 *>(base);
     float *RSG = base + 4 * R.nslot;
     int *RVM = reinterpret_cast<int *>(base + 5 * R.nslot);
+    // rigid texture: the grain maps at the pixels (three arrays), the template's
+    // correction G of the iteration
+    float *RH = base + run_plain_floats(R.nslot), *RTG = RH + 3 * R.nslot;
+    const bool rigid_on = RIGID && A.grain_scal[4] != 0.0;  // uniform: the image has measurable speckle
     const double cx = d.coord[0], cy = d.coord[1];
     const int cxi = (int)cx, cyi = (int)cy;
     const double fxd = floor(cx), fyd = floor(cy);
@@ -554,6 +569,22 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         }
         run_warp_sums<3 * NMOM, (NMOM > 1)>(mom, sm.part[wid], sm.red2[wid] + NVA, lane);
     }
+    if constexpr (RIGID) {
+        if (rigid_on) {
+#pragma unroll 1
+            for (int t = tid; t < T; t += NT) {
+                int dx, dy0;
+                unpack_task(tasks[t], dx, dy0);
+#pragma unroll 1
+                for (int j = 0; j < K; j++) {
+                    float hv[3];
+                    grain_sample(A.grain, A.h, A.w, cx + (double)dx, cy + (double)(dy0 + j), hv);
+#pragma unroll
+                    for (int m = 0; m < 3; m++) RH[m * R.nslot + j * T + t] = hv[m];
+                }
+            }
+        }
+    }
     __syncthreads();
     constexpr int NV = NVA + 3 * NMOM;
     if (wid == 0) {
@@ -656,6 +687,83 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         const uint32_t o0 = 0u - kMagicBits * ((uint32_t)gP + 1u);
         const float2 O2 = make_float2(oy - half, ox - half), U1 = make_float2(vx, ux), U2 = make_float2(vy, uy);
         const float2 Q1 = make_float2(vxx, uxx), Q2 = make_float2(vxy, uxy), C2 = make_float2(vyy, uyy);
+        if constexpr (RIGID) {
+            if (rigid_on) {
+                // Template pass: G(E(p)) per pixel (grain_template,
+                // src/texture.rs:213-244), zero outside the template, and the
+                // sums of G, G^2, (f - f_m) G and SDI_j G.  The template's mean,
+                // spread and gradient are the setup's fixed FP64 sums plus
+                // these, which scale with the strain, so their FP32 rounding
+                // vanishes with it.
+                const float s2f = (float)A.grain_scal[2], fmsf = (float)((double)shift - fm);
+                const float2 px2 = make_float2(ORDER == 2 ? (float)sm.p[6 % M] : 0.f, ORDER == 2 ? (float)sm.p[7 % M] : 0.f);
+                const float2 pxy = make_float2(ORDER == 2 ? (float)sm.p[8 % M] : 0.f, ORDER == 2 ? (float)sm.p[9 % M] : 0.f);
+                const float2 py2 = make_float2(ORDER == 2 ? (float)sm.p[10 % M] : 0.f, ORDER == 2 ? (float)sm.p[11 % M] : 0.f);
+                double g1 = 0.0, g2 = 0.0, gf = 0.0;
+                KSum unused[3];
+                float2 TB[6];
+#pragma unroll
+                for (int k = 0; k < 6; k++) TB[k] = make_float2(0.f, 0.f);
+#pragma unroll 1
+                for (int t = tid; t < T; t += NT) {
+                    int dx, dy0;
+                    unpack_task(tasks[t], dx, dy0);
+                    const float dxf = (float)dx;
+                    RunAcc ac;
+                    ac.p1 = ac.p2 = ac.pfg = 0.f;
+                    ac.m0 = ac.m1 = ac.m2 = make_float2(0.f, 0.f);
+                    // the run's records and grain samples together in flight (the
+                    // stores of G below would order the loads after them)
+                    float4 rcs[K];
+                    float hs[K][3];
+#pragma unroll
+                    for (int j = 0; j < K; j++) {
+                        rcs[j] = ld_rec(REC + j * T + t);
+#pragma unroll
+                        for (int m = 0; m < 3; m++) hs[j][m] = ld_once(RH + m * R.nslot + j * T + t);
+                    }
+#pragma unroll
+                    for (int j = 0; j < K; j++) {
+                        const int sl = j * T + t;
+                        float4 rc = rcs[j];
+                        const float h0 = hs[j][0], h1 = hs[j][1], h2 = hs[j][2];
+                        const float dyf = (float)(dy0 + j);
+                        // (u, v) gradients along x and y at the pixel
+                        float gux = ux, gvx = vx, guy = uy, gvy = vy;
+                        if (ORDER == 2) {
+                            gux = fmaf(px2.x, dxf, fmaf(pxy.x, dyf, ux));
+                            gvx = fmaf(px2.y, dxf, fmaf(pxy.y, dyf, vx));
+                            guy = fmaf(pxy.x, dxf, fmaf(py2.x, dyf, uy));
+                            gvy = fmaf(pxy.y, dxf, fmaf(py2.y, dyf, vy));
+                        }
+                        float e0, e1, e2;
+                        green_lagrange(gux, gvx, guy, gvy, e0, e1, e2);
+                        rc.z += fmsf;  // f - f_m
+                        const float G = (-0.5f * s2f * (e0 * h0 + e1 * h1 + 2.0f * e2 * h2) - (e0 + e1) * rc.z) * rc.w;
+                        RTG[sl] = G;
+                        acc_sample<ORDER, false>(ac, unused, rc, G, 0.f, make_float2(dyf, dyf), make_float2(dyf * dyf, dyf * dyf));
+                    }
+                    g1 += (double)ac.p1;
+                    g2 += (double)ac.p2;
+                    gf += (double)ac.pfg;
+                    acc_expand<ORDER>(ac, dxf, TB);
+                }
+                double *dst = sm.red2[wid];
+                const double gv[3] = {g1, g2, gf};
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    const double t = warp_sum(gv[q]);
+                    if (lane == q) dst[q] = t;
+                }
+                float tb[M];
+#pragma unroll
+                for (int j = 0; j < M / 2; j++) {
+                    tb[2 * j] = TB[j].x;
+                    tb[2 * j + 1] = TB[j].y;
+                }
+                run_warp_sums<M, false>(tb, sm.part[wid], dst + 3, lane);
+            }
+        }
         double s1 = 0.0, s2 = 0.0, sfg = 0.0;
         KSum ks[3];
         float2 PB[6];
@@ -689,7 +797,8 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 float2 dy2 = make_float2((float)dy0, (float)dy0);
 #pragma unroll
                 for (int j = 0; j < K; j++) {
-                    const float4 rc = ld_rec(rec);
+                    float4 rc = ld_rec(rec);
+                    if (RIGID && rigid_on) rc.z += ld_once(RTG + j * T + t);  // the cross term against the template
                     float2 L = A2;
                     const float2 dd2 = __fmul2_rn(dy2, dy2);
                     if (ORDER >= 1) L = __ffma2_rn(B2, dy2, L);
@@ -744,7 +853,9 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                         g = contract<float>(A.g32 + (int64_t)(iy + B - 2) * A.pitch32 + (ix + B - 2), A.pitch32, a, b);
                     }
                     const int sl = j * T + t;
-                    acc_sample<ORDER, KAHAN>(ac, ks, REC[sl], g, fmf, make_float2(dyf, dyf), make_float2(dyf * dyf, dyf * dyf));
+                    float4 rc = REC[sl];
+                    if (RIGID && rigid_on) rc.z += RTG[sl];
+                    acc_sample<ORDER, KAHAN>(ac, ks, rc, g, fmf, make_float2(dyf, dyf), make_float2(dyf * dyf, dyf * dyf));
                 }
             }
             if (!KAHAN) {
@@ -791,14 +902,31 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             const double dg2p = dg2 > 0.0 ? dg2 : 0.0;
             // sum (f - f_m)(g - g_m) = sum (f - f_m)(g - f_m) (sum (f - f_m) = 0)
             //                     = sum (f - s)(g - f_m) - (f_m - s) sum (g - f_m)
-            const double sab = t2 - (fm - (double)shift) * t0;
+            double sab = t2 - (fm - (double)shift) * t0;
+            double dref = df, inv_dref = inv_df, tmf = 0.0, sgj = 0.0;
+            if constexpr (RIGID) {
+                if (rigid_on) {  // against the template t = f + G: t_m = f_m + tmf, spread dref
+                    double tq = 0.0;
+                    if (lane < KR) {
+#pragma unroll
+                        for (int w = 0; w < NT / 32; w++) tq += sm.red2[w][lane];
+                    }
+                    const double q0 = __shfl_sync(0xffffffffu, tq, 0), q1 = __shfl_sync(0xffffffffu, tq, 1);
+                    const double q2 = __shfl_sync(0xffffffffu, tq, 2);
+                    sgj = __shfl_down_sync(0xffffffffu, tq, 3);  // lane j: sum SDI_j G
+                    tmf = q0 * inv_dn;
+                    dref = sqrt(fmax(saa + 2.0 * q2 + q1 - q0 * tmf, 0.0));
+                    inv_dref = 1.0 / dref;
+                    sab -= tmf * t0;
+                }
+            }
             const double rdg = rsqrt(dg2p);  // 1 / delta_g: one reciprocal square root on the update's critical path
             const double dg = dg2p > 0.0 ? dg2p * rdg : 0.0;
-            const double znssd = 2.0 - 2.0 * sab * (inv_df * rdg);
-            const double ratio = df * rdg;
+            const double znssd = 2.0 - 2.0 * sab * (inv_dref * rdg);
+            const double ratio = dref * rdg;
             // lane j < M: grad_j = A_j - (df/dg)(B_j - g~_m S_j); B_j sits at lane 3 + j
             const double bj = __shfl_down_sync(0xffffffffu, tl, 3);
-            const double gj = lane < M ? sm.A[lane] - ratio * (bj - gmt * sm.S[lane]) : 0.0;
+            const double gj = lane < M ? sm.A[lane] + (RIGID ? sgj - tmf * sm.S[lane] : 0.0) - ratio * (bj - gmt * sm.S[lane]) : 0.0;
             // dp = -H^-1 grad with the inverse formed from the Cholesky factor at setup
             // (12 lanes, two FMA chains each; 1.7% faster than two substitutions)
             if (lane < M) sm.grad[lane] = gj;
@@ -848,6 +976,8 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 sm.misc[2] = gmt;
                 sm.misc[3] = dg;
                 sm.misc[4] = znssd;
+                sm.misc[8] = tmf;  // the template's mean less f_m, and its spread (the diagnostic)
+                sm.misc[9] = dref;
             }
         }
         __syncthreads();
@@ -873,8 +1003,9 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     const bool want_eta = ETA && iters > 0 && status == GPV_OK;
     if constexpr (ETA) {
         if (want_eta)
-            run_eta<ORDER, NT, K>(sm, win, A.g32, A.pitch32, A.w, A.h, B, tasks, T, REC, RSG, RVM, cx, cy, (double)shift - fm,
-                              dn, df, gm_last, dg_last, &eu, &ev);
+            run_eta<ORDER, NT, K>(sm, win, A.g32, A.pitch32, A.w, A.h, B, tasks, T, REC, RSG, RVM, rigid_on ? RTG : nullptr, cx,
+                                  cy, (double)shift - fm - (rigid_on ? sm.misc[8] : 0.0), dn, rigid_on ? sm.misc[9] : df,
+                                  gm_last, dg_last, &eu, &ev);
     }
     if (tid == 0) {
         gpv_subset_result *o = A.out + idx;
@@ -895,7 +1026,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         o->status = status;
         o->n_px = n;
         o->has_eta = want_eta;
-        o->texture = 0;
+        o->texture = rigid_on ? 1 : 0;
         o->reserved = 0;
     }
 }
@@ -922,7 +1053,7 @@ __device__ int run_claim_slot(const RunArgs &R) {
 // PER_SUBSET: one block per subset with a claimed scratch slot (subsets
 // free SMs one at a time, for callers sharing the GPU); else a persistent
 // grid whose blocks take subsets of their segment from the queue.
-template <int ORDER, int NT, int K, bool PER_SUBSET, bool KAHAN, bool ETA>
+template <int ORDER, int NT, int K, bool PER_SUBSET, bool KAHAN, bool ETA, bool RIGID>
 __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
     extern __shared__ float4 win4[];
     float *win = reinterpret_cast<float *>(win4);
@@ -946,7 +1077,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
         if (d.radius < 1 || d.radius > A.max_radius) {
             if (threadIdx.x == 0) write_failed(A, idx, d, 12, GPV_INVALID_SUBSET, 0, 0.0, 0.0);
         } else {
-            run_subset<ORDER, NT, K, KAHAN, ETA>(R, idx, d, base, win, sm);
+            run_subset<ORDER, NT, K, KAHAN, ETA, RIGID>(R, idx, d, base, win, sm);
         }
         __threadfence();  // every scratch access of the block is done before the slot is free
         __syncthreads();
@@ -969,26 +1100,33 @@ __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
             if (threadIdx.x == 0) write_failed(A, idx, d, 12, GPV_INVALID_SUBSET, 0, 0.0, 0.0);
             continue;
         }
-        run_subset<ORDER, NT, K, KAHAN, ETA>(R, idx, d, base, win, sm);
+        run_subset<ORDER, NT, K, KAHAN, ETA, RIGID>(R, idx, d, base, win, sm);
     }
 }
 
 // Instantiations: every (threads, one block per subset, with or without the
-// diagnostic); the compensated-sum form on persistent grids of 128 or 256
-// threads only.
+// diagnostic); the compensated-sum form and the rigid-texture template (orders
+// 1 and 2) on persistent grids of 128 or 256 threads only.
 template <int NT, bool PS, bool KH, bool ETA>
 const void *run_kernel_t(int order) {
-    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, PS, KH, ETA>
-                      : (order == 1 ? (const void *)icgn_runs<1, NT, kRunK, PS, KH, ETA>
-                                    : (const void *)icgn_runs<0, NT, kRunK, PS, KH, ETA>);
+    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, PS, KH, ETA, false>
+                      : (order == 1 ? (const void *)icgn_runs<1, NT, kRunK, PS, KH, ETA, false>
+                                    : (const void *)icgn_runs<0, NT, kRunK, PS, KH, ETA, false>);
+}
+
+template <int NT, bool ETA>
+const void *run_kernel_rigid(int order) {
+    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, false, false, ETA, true>
+                      : (const void *)icgn_runs<1, NT, kRunK, false, false, ETA, true>;
 }
 
 template <int NT>
-const void *run_kernel_nt(int order, bool ps, bool kahan, bool eta) {
+const void *run_kernel_nt(int order, RunForm form, bool eta) {
     if constexpr (NT >= 128) {
-        if (kahan) return eta ? run_kernel_t<NT, false, true, true>(order) : run_kernel_t<NT, false, true, false>(order);
+        if (form == RunForm::kRigid) return eta ? run_kernel_rigid<NT, true>(order) : run_kernel_rigid<NT, false>(order);
+        if (form == RunForm::kKahan) return eta ? run_kernel_t<NT, false, true, true>(order) : run_kernel_t<NT, false, true, false>(order);
     }
-    if (ps) return eta ? run_kernel_t<NT, true, false, true>(order) : run_kernel_t<NT, true, false, false>(order);
+    if (form == RunForm::kPerSubset) return eta ? run_kernel_t<NT, true, false, true>(order) : run_kernel_t<NT, true, false, false>(order);
     return eta ? run_kernel_t<NT, false, false, true>(order) : run_kernel_t<NT, false, false, false>(order);
 }
 
@@ -1057,19 +1195,20 @@ int run_window_cap(int rmax) {
 }
 
 // Record slots per block (largest radius's runs x kRunK, rounded to 32) and the
-// scratch floats per block: a float4 record and an eta resample per slot +
-// one validity word per task.
-int64_t run_scratch_floats(gpv_context *ctx, int rmax, int *nslot) {
-    int T = 0;  // the most tasks of any radius up to rmax (the count is not monotone in r)
+// scratch floats per block: a float4 record and an eta resample per slot, one
+// word of pixel bits per run; for the rigid template three grain samples and
+// the correction per slot.
+int64_t run_scratch_floats(gpv_context *ctx, int rmax, bool rigid, int *nslot) {
+    int T = 0;  // the most runs of any radius up to rmax (the count is not monotone in r)
     for (int r = 1; r <= rmax; r++) T = std::max(T, (int)ctx->h_run_n[r]);
     const int ns = (T * kRunK + 31) / 32 * 32;
     *nslot = ns;
-    return 5 * (int64_t)ns + (T + 31) / 32 * 32;
+    return run_plain_floats(ns) + (rigid ? 4 * (int64_t)ns : 0);
 }
 
-const void *run_kernel(int order, int nt, bool per_subset, bool kahan, bool eta) {
-    if (nt == 64) return run_kernel_nt<64>(order, per_subset, kahan, eta);
-    return nt == 256 ? run_kernel_nt<256>(order, per_subset, kahan, eta) : run_kernel_nt<128>(order, per_subset, kahan, eta);
+const void *run_kernel(int order, int nt, RunForm form, bool eta) {
+    if (nt == 64) return run_kernel_nt<64>(order, form, eta);
+    return nt == 256 ? run_kernel_nt<256>(order, form, eta) : run_kernel_nt<128>(order, form, eta);
 }
 
 int run_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,

@@ -28,6 +28,12 @@ struct RunArgs {
     int slots_per_sm, n_mask;
 };
 
+// Scratch floats of a block without the rigid template's part: float4 records,
+// the diagnostic's samples, the runs' pixel bits (nslot / kRunK runs at most).
+__host__ __device__ __forceinline__ int64_t run_plain_floats(int nslot) {
+    return 5 * (int64_t)nslot + (nslot / kRunK + 31) / 32 * 32;
+}
+
 // The context's run tables (ensure_run_tables).
 inline void run_tables(const gpv_context *ctx, RunArgs &R) {
     const int32_t *t = static_cast<const int32_t *>(ctx->run_tab.ptr);

@@ -215,30 +215,6 @@ __device__ __forceinline__ void unpack_off(float w, float &dx, float &dy) {
     dy = (float)(v >> 16);
 }
 
-// The three grain maps (fxx, fyy, fxy; rows x cols FP32) at (x = column,
-// y = row), bilinear, clamped (GrainMaps::sample, src/texture.rs:125-143).
-__device__ __forceinline__ void grain_sample(const float *maps, int rows, int cols, double x, double y, float h[3]) {
-    x = fmin(fmax(x, 0.0), (double)(cols - 1));
-    y = fmin(fmax(y, 0.0), (double)(rows - 1));
-    const int x0 = min((int)floor(x), max(cols - 2, 0)), y0 = min((int)floor(y), max(rows - 2, 0));
-    const int x1 = min(x0 + 1, cols - 1), y1 = min(y0 + 1, rows - 1);
-    const double tx = x - (double)x0, ty = y - (double)y0;
-    const int64_t np = (int64_t)rows * cols;
-#pragma unroll
-    for (int m = 0; m < 3; m++) {
-        const float *M = maps + m * np;
-        h[m] = (float)((1.0 - ty) * ((1.0 - tx) * M[(int64_t)y0 * cols + x0] + tx * M[(int64_t)y0 * cols + x1]) +
-                       ty * ((1.0 - tx) * M[(int64_t)y1 * cols + x0] + tx * M[(int64_t)y1 * cols + x1]));
-    }
-}
-
-// Green-Lagrange strain [Exx, Eyy, Exy] (src/texture.rs:200-206).
-__device__ __forceinline__ void green_lagrange(float ux, float vx, float uy, float vy, float &e0, float &e1, float &e2) {
-    e0 = ux + 0.5f * (ux * ux + vx * vx);
-    e1 = vy + 0.5f * (uy * uy + vy * vy);
-    e2 = 0.5f * (uy + vx) + 0.5f * (ux * uy + vx * vy);
-}
-
 // RIGID: the rigid-texture template (Texture::Rigid) when the reference image
 // has measurable speckle: the maps at the subset pixels in setup (Sh: 3
 // arrays of n_max), and every iteration a template pass storing the
@@ -1343,7 +1319,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             P.smem = sizeof(double) * (size_t)P.cap;
             GPV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&P.per_sm, P.fn, P.nt, P.smem));
             if (P.per_sm < 1) { set_error("subset window does not fit in shared memory"); return GPV_ERR_INVALID; }
-            run_scratch_floats(ctx, P.rmax, &P.nslot);
+            run_scratch_floats(ctx, P.rmax, false, &P.nslot);
             P.stride = 2 * run64_scratch_doubles(P.nslot, fagn);  // floats
             P.blocks = (int)std::min<int64_t>((int64_t)P.per_sm * ctx->num_sms, n);
             region = std::max(region, P.blocks * P.stride);
@@ -1356,15 +1332,16 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
         // GPV_SOLVE_KAHAN (compensated FP64 ZNSSD sums): run-layout
         // kernel on a persistent grid
         const bool kahan = (K.flags & GPV_SOLVE_KAHAN) != 0;
-        P.runs = !P.rigid && (use_run_kernel() || kahan);
+        P.runs = use_run_kernel() || (kahan && !P.rigid);
         if (kahan) P.ps = false;
         if (P.runs) {
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
         }
         P.cap = P.runs ? run_window_cap(P.rmax) : window_cap(P.rmax, P.layout);
         // 64-thread blocks exist for the run-layout kernel (not its compensated form) only
-        if (P.nt == 64 && (!P.runs || kahan)) P.nt = 128;
-        const void *fn = P.runs ? run_kernel(order, P.nt, P.ps, kahan, (K.flags & GPV_SOLVE_ETA) != 0)
+        if (P.nt == 64 && (!P.runs || kahan || P.rigid)) P.nt = 128;
+        const RunForm rf = P.rigid ? RunForm::kRigid : (kahan ? RunForm::kKahan : (P.ps ? RunForm::kPerSubset : RunForm::kPlain));
+        const void *fn = P.runs ? run_kernel(order, P.nt, rf, (K.flags & GPV_SOLVE_ETA) != 0)
                                 : tile_kernel(P.nt, P.ps, order, P.rigid);
         P.fn = fn;
         int max_bytes = 0;
@@ -1393,7 +1370,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
         P.per_sm = per_sm;
         const int64_t nmax = (int64_t)(ctx->h_slot_n[P.rmax] + 31) / 32 * 32;
         P.stride = (P.rigid ? 9 : 5) * nmax;  // float4 record + eta sample (+ 3 grain samples, template) per pixel
-        if (P.runs) P.stride = run_scratch_floats(ctx, P.rmax, &P.nslot);
+        if (P.runs) P.stride = run_scratch_floats(ctx, P.rmax, P.rigid, &P.nslot);
         int64_t slots;
         if (P.ps) {
             P.blocks = (int)ctx->seg_count[q];

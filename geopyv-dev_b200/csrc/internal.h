@@ -206,8 +206,9 @@ int query_nsmid(int *out);
 // time, runs of four template pixels per lane)
 int ensure_run_tables(gpv_context *ctx, int max_radius);
 int run_window_cap(int rmax);
-int64_t run_scratch_floats(gpv_context *ctx, int rmax, int *nslot);
-const void *run_kernel(int order, int nt, bool per_subset, bool kahan, bool eta);
+int64_t run_scratch_floats(gpv_context *ctx, int rmax, bool rigid, int *nslot);
+enum class RunForm { kPlain, kPerSubset, kKahan, kRigid };
+const void *run_kernel(int order, int nt, RunForm form, bool eta);
 struct KArgs;
 int run_launch(gpv_context *ctx, const void *fn, int nt, int blocks, size_t smem, cudaStream_t s, const KArgs &k,
                const int32_t *seg, int *queue, int win_cap, int nslot, uint32_t *slot_mask, int slots_per_sm, int n_mask);

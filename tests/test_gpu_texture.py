@@ -76,6 +76,34 @@ def test_rigid_solve_matches_the_oracle(gpv_mod, oracle, order, gamma):
 
 
 @pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("radius", [16, 33, 45])
+def test_rigid_run_layout_matches_the_oracle(gpv_mod, oracle, radius, order):
+    """More subsets than SMs (128 threads each, 256 above radius 40), bands of
+    four rows with and without a remainder, some subsets over the image's edge
+    (the clamped path), against the oracle within the mixed bar.  Two subsets
+    of radius 45, half outside the image, diverge at second order in the oracle
+    too: they need not end in the same iteration, only unconverged."""
+    gamma = 0.05
+    f, g = TC.shear_pair(gamma)
+    d = np.concatenate([TC.grid_desc(gpv_mod, gamma, order)] * 9)
+    d["radius"] = radius
+    d["coord"][::7, 0] -= 30.0  # over the left edge for the larger radii
+    kw = dict(max_norm=1e-5, max_iterations=100, tolerance=0.75)
+    maps, s2 = oracle.grain(f)
+    cf, cg = oracle.get_c(f, 8), oracle.get_c(g, 8)
+    ref = oracle.solve_batch(cf, cg, f.shape, 8, d, grain=(maps, s2), eta=True, **kw)
+    F, G = gpv_mod.Image(image_gs=f, border=8), gpv_mod.Image(image_gs=g, border=8)
+    r = gpv_mod.solve_batch(F, G, d, texture="rigid", eta=True, **kw)
+    assert np.all(r["texture"] == 1) and np.array_equal(r["converged"], ref["converged"])
+    ok = (ref["status"] == 0) & (ref["converged"] == 1)
+    assert ok.any() and np.array_equal(r["status"][ok], ref["status"][ok])
+    assert np.abs(r["p"][ok, :2] - ref["p"][ok, :2]).max() <= 1e-3
+    assert np.abs(r["p"][ok, 2:6] - ref["p"][ok, 2:6]).max() <= 1e-5
+    assert np.abs(r["c_zncc"][ok] - ref["c_zncc"][ok]).max() < 1e-5
+    assert np.abs(r["eta_u"][ok] - ref["eta_u"][ok]).max() < 2e-3
+
+
+@pytest.mark.parametrize("order", [1, 2])
 def test_rigid_fagn_matches_the_oracle(gpv_mod, oracle, order):
     """FAGN with the rigid template (src/subset.rs:1228-1334), FP64 arithmetic:
     on FP64 coefficients (and FP64 grain maps) within 1e-8 px of the oracle,
