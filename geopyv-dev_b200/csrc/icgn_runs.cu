@@ -407,9 +407,13 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     // under the centre: keeps the sums free of cancellation and a flat
     // subset's sums exactly zero); FP32 per thread, FP64 across the block.
     constexpr int NVA = 4 + 2 * M;
+    // 64 threads have twice the runs each: their FP32 sums are taken in halves,
+    // so that no more pixels than with 128 threads share one (the error of
+    // delta_f and of the ZNCC against 64 bits would be 1.5 to 2.5 times as large)
+    constexpr int kHalves = NT == 64 ? 2 : 1;
+    const int t_half = kHalves == 2 ? (T + 2 * NT - 1) / (2 * NT) * NT : T;
+    double carry = 0.0;
     float acc[NVA];
-#pragma unroll
-    for (int q = 0; q < NVA; q++) acc[q] = 0.f;
     float shift;
     if (f_staged) {
         const int wx = min(max(max(0, min(bx, A.w - 1)) + B - fc0, 0), fww - 1);
@@ -446,7 +450,12 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             bb[k] = make_float2(b0[k], b0[k]);
             dbb[k] = make_float2(db0[k], db0[k]);
         }
-        for (int t = tid; t < T; t += NT) {
+#pragma unroll 1
+        for (int hf = 0; hf < kHalves; hf++) {
+#pragma unroll
+        for (int q = 0; q < NVA; q++) acc[q] = 0.f;
+        const int t_end = kHalves == 2 ? min(T, (hf + 1) * t_half) : T;
+        for (int t = kHalves == 2 ? hf * t_half + tid : tid; t < t_end; t += NT) {
             int dx, dy0;
             unpack_task(tasks[t], dx, dy0);
             uint32_t vm = (uint32_t)tasks[t].y;
@@ -523,8 +532,18 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 }
             }
         }
+        run_warp_sums<NVA, (NVA > 16)>(acc, sm.part[wid], sm.red2[wid], lane);
+        if constexpr (kHalves == 2) {
+            static_assert(NVA <= 32, "one sum per lane");
+            __syncwarp();
+            if (lane < NVA) {
+                carry += sm.red2[wid][lane];
+                sm.red2[wid][lane] = carry;
+            }
+            __syncwarp();
+        }
+        }
     }
-    run_warp_sums<NVA, (NVA > 16)>(acc, sm.part[wid], sm.red2[wid], lane);
     // ---- setup, pass 2: the Hessian's gradient moments ----------------------
     // sum g_p g_q dx^a dy^b (a + b <= 2 DEG) per run as powers of dy, then
     // expanded by the run's powers of dx; each thread re-reads its own records
@@ -767,8 +786,10 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         double s1 = 0.0, s2 = 0.0, sfg = 0.0;
         KSum ks[3];
         float2 PB[6];
+        float2 PH[6];  // 64 threads: pairs of runs are added first (as the setup's halves)
+        bool pair = false;
 #pragma unroll
-        for (int k = 0; k < 6; k++) PB[k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < 6; k++) PB[k] = PH[k] = make_float2(0.f, 0.f);
         for (int t = tid; t < T; t += NT) {
             int dx, dy0;
             unpack_task(tasks[t], dx, dy0);
@@ -787,9 +808,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             ac.m0 = ac.m1 = ac.m2 = make_float2(0.f, 0.f);
             if (fast) {
                 // no edge clamp can apply and the window covers every tap: the
-                // block of coefficients rolls down the run in registers, two
-                // samples per pass of a rolled loop (seven rows held; the last
-                // five move up two places between passes)
+                // block of coefficients rolls down the run in registers
                 float Rg[6][6];
                 int py = 0, px = 0;  // floors of the sample before (biased)
                 uint32_t off = o0 + (uint32_t)((dy0 + wy0) * gP + dx + wx0);
@@ -863,7 +882,23 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 s2 += (double)ac.p2;
                 sfg += (double)ac.pfg;
             }
-            acc_expand<ORDER>(ac, dxf, PB);
+            if constexpr (NT == 64) {
+                acc_expand<ORDER>(ac, dxf, PH);
+                if (pair) {
+#pragma unroll
+                    for (int k = 0; k < M / 2; k++) {
+                        PB[k] = __fadd2_rn(PB[k], PH[k]);
+                        PH[k] = make_float2(0.f, 0.f);
+                    }
+                }
+                pair = !pair;
+            } else {
+                acc_expand<ORDER>(ac, dxf, PB);
+            }
+        }
+        if constexpr (NT == 64) {
+#pragma unroll
+            for (int k = 0; k < M / 2; k++) PB[k] = __fadd2_rn(PB[k], PH[k]);
         }
         // block sums: warp partials to shared memory, one barrier, then warp 0
         // adds them up and updates the warp; a second barrier publishes p

@@ -1282,7 +1282,7 @@ bool use_run_kernel();
 // Threads per block of the tiled kernel for subsets of radius r: the
 // autotuned choice when one was recorded for this radius class, else a
 // size rule (GPV_TILE_THREADS overrides).
-int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n);
+int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n);
 
 // Raise a kernel's dynamic shared-memory limit to everything the device
 // allows beside its static shared memory, once per (device, kernel).  The
@@ -1413,7 +1413,7 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             region = std::max(region, P.blocks * P.stride);
             continue;
         }
-        P.nt = tile_threads_for(ctx, P.rmax, n);
+        P.nt = tile_threads_for(ctx, order, P.rmax, n);
         P.layout = tile_layout_for(ctx, P.rmax);
         // persistent deformable segments run the run-layout kernel unless
         // GPV_SOLVE_KERNEL=tile asks for the tiled one
@@ -1544,7 +1544,7 @@ bool use_run_kernel() {
     return !(v && v[0] == 't');
 }
 
-int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n) {
+int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n) {
     if (ctx->force_threads) return ctx->force_threads;
     if (const char *v = getenv("GPV_TILE_THREADS")) {
         const int t = atoi(v);
@@ -1558,6 +1558,16 @@ int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n) {
     if (n <= ctx->num_sms) return 256;
     const int cls = max_radius <= 20 ? 0 : (max_radius <= 40 ? 1 : 2);
     if (ctx->tuned_threads[cls]) return ctx->tuned_threads[cls];
+    // 64 threads, eight subsets per SM: one subset's serial part (sums, update)
+    // passes behind seven others' samples, while their windows still share the
+    // SM.  Times of 128 over 64 threads: first order, radius 18 1.05, 25 1.02,
+    // 28 0.97-1.02, 30 (windows over an eighth of the SM) 0.66-0.78; order 0,
+    // radius 16 1.03-1.05, 25 1.05-1.09; second order, radius 8 1.28, 12 1.14,
+    // 14 1.12 (64 threads also leave fewer lanes idle in the last round of its
+    // runs), 16 0.98, 20 0.99.  Below one and a half rounds of 1,184 subsets the
+    // last round weighs more (first order, radius 25: 1,444 subsets 0.95, 1,849
+    // 1.01).
+    if (n >= 12 * (int64_t)ctx->num_sms && max_radius <= (order == 2 ? 14 : 25)) return 64;
     return max_radius > 40 ? 256 : 128;
 }
 

@@ -71,6 +71,38 @@ def test_batch_matches_oracle(oracle, gpv_mod, config, scale, precision):
     assert np.median(err) < 0.05
 
 
+@pytest.mark.parametrize("eta", [False, True])
+@pytest.mark.parametrize("order,radius", [(0, 9), (0, 25), (1, 9), (1, 25), (1, 26), (2, 9), (2, 14), (2, 15)])
+def test_large_batches_of_small_subsets_match_oracle(oracle, gpv_mod, order, radius, eta):
+    """Twelve subsets per SM: 64 threads per subset up to radius 25 (14 at second
+    order), 128 from the next radius on, against the oracle on the distinct
+    subsets within the mixed bar; every copy of a subset gives the same bytes.
+    Iteration counts are left out: with 16 iterations on the average (radius 9,
+    second order) one subset in nine has a norm near max_norm at some iteration,
+    at any number of threads."""
+    import torch
+    from gpv import synth
+    W = synth.workload(2, scale_down=16)
+    F, G, Cf, Cg = _images(gpv_mod, oracle, W)
+    base = _desc(gpv_mod, W)
+    base["radius"], base["order"] = radius, order
+    base["p0"][:, (2, 6, 12)[order]:] = 0.0
+    n = 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    d = base[np.arange(n) % len(base)]
+    kw = dict(max_norm=1e-5, max_iterations=50, tolerance=0.75, eta=eta)
+    ref = oracle.solve_batch(Cf, Cg, W["f"].shape, BORDER, base, **kw)
+    res = gpv_mod.solve_batch(F, G, d, **kw)
+    m = min(n, len(base))
+    first = res[:m].copy()
+    res["iterations"][:m] = ref["iterations"][:m]
+    _compare(res[:m], ref[:m], False, f"order {order} radius {radius}")
+    if eta:
+        ok = ref["status"][:m] == 0
+        assert np.abs(res["eta_u"][:m][ok] - ref["eta_u"][:m][ok]).max() < 2e-3
+    for k in range(m, n, m):
+        assert res[k:k + m].tobytes() == first[:min(m, n - k)].tobytes()
+
+
 @pytest.mark.parametrize("config,scale", [(2, 16), (3, 8)])
 def test_compensated_sums_match_oracle(oracle, gpv_mod, config, scale):
     """The Kahan-compensated FP64 ZNSSD sums (GPV_SOLVE_KAHAN) meet the
