@@ -45,15 +45,17 @@
 //    radius 25 2.35 -> 2.18 ms; the shared cache 67 % busy.  A pool of 16 warps per
 //    SM sharing five subsets (no block barriers) measured 2.6 times slower: its
 //    warps fetch each stretch alone, at 93 % of that cache.
-//  * Sums.  The per-iteration sums (g - f_m, its square, (f - f_m)(g - f_m)
-//    and the steepest-descent products) are FP32 over one run (at most K
-//    samples), then FP64 per thread and across the block in a fixed order
-//    (deterministic).
+//  * Sums.  The per-iteration sums g - f_m, its square and (f - f_m)(g - f_m)
+//    are FP32 over one run (at most K samples), then FP64 per thread and across
+//    the block in a fixed order (deterministic); the steepest-descent products
+//    and the setup's sums are FP32 per thread, then FP64.  64 threads take these
+//    in pairs of runs and in halves, as many terms as 128 threads have.
 //  * Rigid texture (RIGID; orders 1 and 2): the grain maps sampled per pixel at
 //    setup, and a template pass per iteration with the sums of its correction G
 //    (the run's four pixels' loads together in flight); the sample loop only adds
 //    G to its cross term.  14,420 second-order subsets of radius 30 4.33 ms in the
-//    tiled kernel, 3.2 here (deformable 2.0).
+//    tiled kernel, 3.2 here (deformable 2.0).  With the diagnostic the tiled
+//    kernel stays: see the launcher.
 // Subsets whose warped square leaves the image or the staged window take a
 // clamped per-sample path (the reference's edge clamp, src/image.rs:129-132),
 // reading the window with clamped indices or global memory.
@@ -296,7 +298,7 @@ __device__ __forceinline__ void acc_expand(const RunAcc &a, float dxf, float2 (&
 template <int ORDER, int NT, int K>
 __device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, const float *__restrict__ g32, int64_t pitch32,
                                      int w, int h, int B, const int2 *tasks, int T, const float4 *REC, float *RSG,
-                                     const int *RVM, const float *RTG, double cx, double cy, double fms, double dn, double df, double gm,
+                                     const int *RVM, double cx, double cy, double fms, double dn, double df, double gm,
                                      double dg, double *eu, double *ev) {
     constexpr int M = Ord<ORDER>::M;
     const int tid = threadIdx.x;
@@ -344,7 +346,7 @@ __device__ __forceinline__ void run_eta(RunSmem<NT / 32> &sm, const float *win, 
                     }
                 }
                 const float4 rec = REC[sl];
-                fn((double)rec.z + (RTG ? (double)RTG[sl] : 0.0) + fms, (double)rec.x, (double)rec.y, (double)RSG[sl] - gm, dx, dy);
+                fn((double)rec.z + fms, (double)rec.x, (double)rec.y, (double)RSG[sl] - gm, dx, dy);
             }
         }
     };
@@ -701,8 +703,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         // ((y, x) pairs; |s| ~ the fraction plus the deformation over the
         // subset): s is rounded in FP32 at its own small magnitude, and the
         // integer offsets join its floor exactly.
-        // (half a pixel lower on the fast path, where floors come by rounding)
-        const float half = fast ? 0.5f : 0.f;
+        // (half a pixel lower on the fast path, where floors come by rounding;
+        // with the diagnostic the half comes off after: it follows the
+        // parameters' last bits, 1e-8 px of another rounding moved it by 5e-6
+        // of its size)
+        const float half = fast && !ETA ? 0.5f : 0.f;
         const uint32_t o0 = 0u - kMagicBits * ((uint32_t)gP + 1u);
         const float2 O2 = make_float2(oy - half, ox - half), U1 = make_float2(vx, ux), U2 = make_float2(vy, uy);
         const float2 Q1 = make_float2(vxx, uxx), Q2 = make_float2(vxy, uxy), C2 = make_float2(vyy, uyy);
@@ -824,8 +829,10 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                     if (ORDER == 2) L = __ffma2_rn(C2, dd2, L);
                     // L is half a pixel below the position: rounding to
                     // nearest gives its floor, and u = fraction - 1/2
-                    const float2 Mg = __fadd2_rn(L, make_float2(kMagic, kMagic));
-                    const float2 u2 = __fadd2_rn(L, __ffma2_rn(Mg, make_float2(-1.f, -1.f), make_float2(kMagic, kMagic)));
+                    const float2 mh = make_float2(-0.5f, -0.5f);
+                    const float2 Mg = __fadd2_rn(ETA ? __fadd2_rn(L, mh) : L, make_float2(kMagic, kMagic));
+                    float2 u2 = __fadd2_rn(L, __ffma2_rn(Mg, make_float2(-1.f, -1.f), make_float2(kMagic, kMagic)));
+                    if (ETA) u2 = __fadd2_rn(u2, mh);
                     const int iy = __float_as_int(Mg.x), ix = __float_as_int(Mg.y);
                     const float *rp = win + (int)(off + (uint32_t)iy * (uint32_t)gP + (uint32_t)ix);
                     if (j == 0 || ix != px || iy != py) {  // the block did not move down one row: (re)load
@@ -1011,8 +1018,6 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 sm.misc[2] = gmt;
                 sm.misc[3] = dg;
                 sm.misc[4] = znssd;
-                sm.misc[8] = tmf;  // the template's mean less f_m, and its spread (the diagnostic)
-                sm.misc[9] = dref;
             }
         }
         __syncthreads();
@@ -1038,9 +1043,8 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     const bool want_eta = ETA && iters > 0 && status == GPV_OK;
     if constexpr (ETA) {
         if (want_eta)
-            run_eta<ORDER, NT, K>(sm, win, A.g32, A.pitch32, A.w, A.h, B, tasks, T, REC, RSG, RVM, rigid_on ? RTG : nullptr, cx,
-                                  cy, (double)shift - fm - (rigid_on ? sm.misc[8] : 0.0), dn, rigid_on ? sm.misc[9] : df,
-                                  gm_last, dg_last, &eu, &ev);
+            run_eta<ORDER, NT, K>(sm, win, A.g32, A.pitch32, A.w, A.h, B, tasks, T, REC, RSG, RVM, cx, cy, (double)shift - fm,
+                              dn, df, gm_last, dg_last, &eu, &ev);
     }
     if (tid == 0) {
         gpv_subset_result *o = A.out + idx;
@@ -1141,7 +1145,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) icgn_runs(RunArgs R) {
 
 // Instantiations: every (threads, one block per subset, with or without the
 // diagnostic); the compensated-sum form and the rigid-texture template (orders
-// 1 and 2) on persistent grids of 128 or 256 threads only.
+// 1 and 2, without the diagnostic) on persistent grids of 128 or 256 threads only.
 template <int NT, bool PS, bool KH, bool ETA>
 const void *run_kernel_t(int order) {
     return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, PS, KH, ETA, false>
@@ -1149,16 +1153,16 @@ const void *run_kernel_t(int order) {
                                     : (const void *)icgn_runs<0, NT, kRunK, PS, KH, ETA, false>);
 }
 
-template <int NT, bool ETA>
+template <int NT>
 const void *run_kernel_rigid(int order) {
-    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, false, false, ETA, true>
-                      : (const void *)icgn_runs<1, NT, kRunK, false, false, ETA, true>;
+    return order == 2 ? (const void *)icgn_runs<2, NT, kRunK, false, false, false, true>
+                      : (const void *)icgn_runs<1, NT, kRunK, false, false, false, true>;
 }
 
 template <int NT>
 const void *run_kernel_nt(int order, RunForm form, bool eta) {
     if constexpr (NT >= 128) {
-        if (form == RunForm::kRigid) return eta ? run_kernel_rigid<NT, true>(order) : run_kernel_rigid<NT, false>(order);
+        if (form == RunForm::kRigid) return run_kernel_rigid<NT>(order);
         if (form == RunForm::kKahan) return eta ? run_kernel_t<NT, false, true, true>(order) : run_kernel_t<NT, false, true, false>(order);
     }
     if (form == RunForm::kPerSubset) return eta ? run_kernel_t<NT, true, false, true>(order) : run_kernel_t<NT, true, false, false>(order);

@@ -217,7 +217,8 @@ __device__ __forceinline__ void unpack_off(float w, float &dx, float &dy) {
     dy = (float)(v >> 16);
 }
 
-// RIGID: the rigid-texture template (Texture::Rigid) when the reference image
+// RIGID (with the omitted-mode diagnostic, or GPV_SOLVE_KERNEL=tile): the
+// rigid-texture template (Texture::Rigid) when the reference image
 // has measurable speckle: the maps at the subset pixels in setup (Sh: 3
 // arrays of n_max), and every iteration a template pass storing the
 // correction G(E(p)) per pixel (St; the template is t = f + G,
@@ -1282,7 +1283,7 @@ bool use_run_kernel();
 // Threads per block of the tiled kernel for subsets of radius r: the
 // autotuned choice when one was recorded for this radius class, else a
 // size rule (GPV_TILE_THREADS overrides).
-int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n);
+int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n, bool eta);
 
 // Raise a kernel's dynamic shared-memory limit to everything the device
 // allows beside its static shared memory, once per (device, kernel).  The
@@ -1413,14 +1414,18 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
             region = std::max(region, P.blocks * P.stride);
             continue;
         }
-        P.nt = tile_threads_for(ctx, order, P.rmax, n);
+        P.nt = tile_threads_for(ctx, order, P.rmax, n, (K.flags & GPV_SOLVE_ETA) != 0);
         P.layout = tile_layout_for(ctx, P.rmax);
         // persistent deformable segments run the run-layout kernel unless
         // GPV_SOLVE_KERNEL=tile asks for the tiled one
         // GPV_SOLVE_KAHAN (compensated FP64 ZNSSD sums): run-layout
         // kernel on a persistent grid
         const bool kahan = (K.flags & GPV_SOLVE_KAHAN) != 0;
-        P.runs = use_run_kernel() || (kahan && !P.rigid);
+        // The rigid template with the omitted-mode diagnostic stays in the tiled
+        // kernel, 1.3-1.8 times slower: the diagnostic follows the parameters' last
+        // bits, and the run layout's other order of sums moves it by 1-3e-5 of its
+        // size (the parameters by 4e-8).
+        P.runs = (use_run_kernel() && !(P.rigid && (K.flags & GPV_SOLVE_ETA))) || (kahan && !P.rigid);
         if (kahan) P.ps = false;
         if (P.runs) {
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
@@ -1544,7 +1549,7 @@ bool use_run_kernel() {
     return !(v && v[0] == 't');
 }
 
-int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n) {
+int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n, bool eta) {
     if (ctx->force_threads) return ctx->force_threads;
     if (const char *v = getenv("GPV_TILE_THREADS")) {
         const int t = atoi(v);
@@ -1566,8 +1571,10 @@ int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n) {
     // 14 1.12 (64 threads also leave fewer lanes idle in the last round of its
     // runs), 16 0.98, 20 0.99.  Below one and a half rounds of 1,184 subsets the
     // last round weighs more (first order, radius 25: 1,444 subsets 0.95, 1,849
-    // 1.01).
-    if (n >= 12 * (int64_t)ctx->num_sms && max_radius <= (order == 2 ? 14 : 25)) return 64;
+    // 1.01).  Not with the omitted-mode diagnostic (1.03-1.05): it follows the
+    // parameters' last bits, and another split of the sums moves it by 5e-6 of
+    // its size.
+    if (!eta && n >= 12 * (int64_t)ctx->num_sms && max_radius <= (order == 2 ? 14 : 25)) return 64;
     return max_radius > 40 ? 256 : 128;
 }
 
