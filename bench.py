@@ -43,7 +43,7 @@ os.environ.setdefault("CUDA_DEVICE_MAX_CONNECTIONS", "32")
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one full-size
 # second-order solve launch, by kernel (captured separately, not in this run)
-ICGN_C2_DRAM_BYTES = {"icgn_tile<2,128>": 977.85e6, "icgn_runs<2,128,4>": 1136.39e6}
+ICGN_C2_DRAM_BYTES = {"icgn_tile<2,128>": 977.85e6, "icgn_runs<2,128,4>": 7164.95e6}
 
 METRIC = "ICGN subsets/s at <=1e-3 px vs FP64 oracle; p50/p99 served solve latency"
 
@@ -443,7 +443,7 @@ def uneven_leg(device, steps=10):
 
 # ---------------------------------------------------------------------------
 def fp64_leg(W, device, mixed_solve_ms, steps=3):
-    """The plain one-subset-per-block FP64 form (icgn_fp64: FP64 coefficients,
+    """The plain one-subset-per-block FP64 form (icgn_runs64: FP64 coefficients,
     interpolation, sums and solve) on the headline batch, device-resident,
     CUDA events around `steps` solves; beside it the mixed form's solve time
     of the same batch from the headline timing."""
@@ -476,7 +476,7 @@ def fp64_leg(W, device, mixed_solve_ms, steps=3):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / steps
     res = np.frombuffer(out_dev.cpu().numpy().tobytes(), dtype=_lib.RESULT_DTYPE).copy()
-    return {"kernel": "icgn_fp64 (one block of 256 threads per subset, FP64 throughout)", "subsets": n,
+    return {"kernel": "icgn_runs64 (run layout, FP64 throughout)", "subsets": n,
             "solve_ms": ms, "fp64_plain_subsets_per_s": n / (ms * 1e-3),
             "mixed_solve_ms": mixed_solve_ms, "mixed_over_fp64": ms / mixed_solve_ms,
             "iterations_mean": float(res["iterations"].mean()), "converged_frac": float(res["converged"].mean()),
@@ -961,7 +961,7 @@ def run_ours(args, world, rank, local):
     runs = os.environ.get("GPV_SOLVE_KERNEL", "runs")[:1] != "t"
     cls = 0 if max_r <= 20 else (1 if max_r <= 40 else 2)
     if prec != gpv.PREC_MIXED:
-        kernel_name = "icgn_fp64"
+        kernel_name = "icgn_runs64"
     elif runs:
         kernel_name = f"icgn_runs<{2 if args.config == 2 else 'mixed'},{tuned[cls] or 128},{runk[cls] or 4}>"
     else:
