@@ -718,7 +718,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 // sum (e - k b + t d)^2 with sum e = -rho sum b (sum a = 0) and sum e b = sum a b - rho sum b^2
                 const double k = t_fg - rho, td = t_fg * gmt;
                 const double srr = tee + k * (k * tbb - 2.0 * (tab - rho * tbb)) - 2.0 * td * (rho * tb + k * tb) + dn * td * td;
-                znssd = fmax(srr, 0.0) / saa;
+                znssd = (srr < 0.0 ? 0.0 : srr) / saa;  // a NaN (delta_g = 0) stays one
                 const double bj = __shfl_down_sync(0xffffffffu, tl, 4);
                 if (lane < M) sm.grad[lane] = sm.A[lane] - t_fg * (bj - gmt * sm.S[lane]);
                 __syncwarp();
