@@ -25,7 +25,10 @@
 //        ZNSSD    = sum r^2 / delta_f^2,
 //    where sum r^2 follows from sum e^2 and small corrections (k and d go to
 //    zero as the solve converges), so ZNSSD keeps the relative accuracy of the
-//    direct sum.
+//    direct sum.  That costs digits where the target's level is far from c against
+//    its contrast (a first iteration on a target of another brightness, or
+//    one without contrast), or rho far above t: there three more sweeps take the
+//    mean, the spread about it and the direct sums.
 //  * FAGN takes two sweeps: target value and gradient at the warped positions
 //    (kept per pixel), then the Hessian's moments and the residual gradient
 //    about the warped centre.
@@ -49,6 +52,10 @@ namespace gpv {
 namespace {
 
 constexpr int kK = kRunK;
+// The sums about a level are used while they leave the spread all but two of
+// its digits (a target ten times its contrast away from the level), and the
+// residual's sum while the scale of the iteration before is within 32 times the new one.
+constexpr double kLevelDigits = 0.01, kScaleDigits = 32.0 * 32.0;
 
 template <int NW>
 struct Smem64 {
@@ -472,6 +479,10 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         }
         const int wy0 = wby + B - 2 - gr0, wx0 = wbx + B - 2 - gc0;
         const bool fast = staged && inside;
+        // sweeps: 0 about the level of the iteration before; where that level or
+        // rho costs digits, 1 the target's mean (about 0), 2 its spread about the
+        // mean, 3 (ICGN) the sums with both
+        for (int sweep = 0;; sweep++) {
         double sb = 0.0, sbb = 0.0, sab = 0.0, see = 0.0;
         double PB[FAGN ? 2 : M];
 #pragma unroll
@@ -609,7 +620,15 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             // sweep 2: moments of the target's gradient about the warped centre, residual gradient, ZNSSD
             const double s0 = block_sum64<NT>(sb, sm), s1 = block_sum64<NT>(sbb, sm);
             gmt = s0 / dn;
-            dg = sqrt(fmax(s1 - s0 * gmt, 0.0));
+            double dg2 = s1 - s0 * gmt;
+            if (sweep == 2) {
+                gmt = 0.0;
+                dg2 = s1;
+            } else if (sweep == 1 || !(dg2 > kLevelDigits * s1)) {  // the same for all threads
+                cg = sweep ? cg + gmt : 0.0;
+                continue;
+            }
+            dg = sqrt(dg2);
             t_fg = df / dg;
             const double gm = cg + gmt, ratio = dg / df, inv_df = 1.0 / df, inv_dg = 1.0 / dg;
             double mo[NMOM * 3], ac[M + 1];
@@ -671,7 +690,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         __syncthreads();
         if (wid == 0) {
             double dpj = 0.0, znssd;
-            bool ok = true;
+            bool ok = true, again = false;
             if constexpr (FAGN) {
                 for (int q = lane; q < M + 1 + 3 * NMOM; q += 32) {
                     double t = 0.0;
@@ -713,11 +732,22 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 const double tb = __shfl_sync(0xffffffffu, tl, 0), tbb = __shfl_sync(0xffffffffu, tl, 1);
                 const double tab = __shfl_sync(0xffffffffu, tl, 2), tee = __shfl_sync(0xffffffffu, tl, 3);
                 gmt = tb / dn;
-                dg = sqrt(fmax(tbb - tb * gmt, 0.0));
+                double dg2 = tbb - tb * gmt;
+                if (sweep == 0) {
+                    again = !(dg2 > kLevelDigits * tbb && rho * rho * dg2 <= kScaleDigits * saa);
+                } else {
+                    again = sweep < 3;
+                    if (sweep > 1) {  // about the mean itself
+                        gmt = 0.0;
+                        dg2 = tbb;
+                    }
+                }
+                dg = sqrt(dg2);
                 t_fg = df / dg;
                 // sum (e - k b + t d)^2 with sum e = -rho sum b (sum a = 0) and sum e b = sum a b - rho sum b^2
                 const double k = t_fg - rho, td = t_fg * gmt;
-                const double srr = tee + k * (k * tbb - 2.0 * (tab - rho * tbb)) - 2.0 * td * (rho * tb + k * tb) + dn * td * td;
+                const double srr = sweep == 3 ? tee  // rho is t
+                                              : tee + k * (k * tbb - 2.0 * (tab - rho * tbb)) - 2.0 * td * (rho * tb + k * tb) + dn * td * td;
                 znssd = (srr < 0.0 ? 0.0 : srr) / saa;  // a NaN (delta_g = 0) stays one
                 const double bj = __shfl_down_sync(0xffffffffu, tl, 4);
                 if (lane < M) sm.grad[lane] = sm.A[lane] - t_fg * (bj - gmt * sm.S[lane]);
@@ -732,12 +762,16 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     dpj = -(a0 + a1);
                 }
             }
-            if (lane < M) {
+            if (lane < M && !again) {
                 sm.dp[lane] = dpj;
                 sm.pprev[lane] = sm.p[lane];
             }
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0 && again) {
+                sm.flag[1] = 2;
+                sm.misc[2] = gmt;
+                sm.misc[9] = t_fg;
+            } else if (lane == 0) {
                 double dpl[12], pl[12];
 #pragma unroll
                 for (int k = 0; k < 12; k++) {
@@ -773,6 +807,11 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             }
         }
         __syncthreads();
+        if (FAGN || sm.flag[1] < 2) break;
+        if (sweep == 0) cg = 0.0;
+        else if (sweep == 1) cg = sm.misc[2];
+        else rho = sm.misc[9];
+        }
         gm_last = cg + sm.misc[2];
         dg_last = sm.misc[3];
         if (!sm.flag[1]) {  // p keeps the last valid warp

@@ -50,3 +50,62 @@ def test_zero_target_gives_no_correlation(gpv_mod, order):
             assert np.isnan(hist[:, 0, 1:]).all()
         else:
             assert np.all(got["c_zncc"] == 0.0) and np.all(got["c_znssd"] == 4.0)
+
+
+@pytest.mark.parametrize("method", ["icgn", "fagn"])
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_target_without_contrast_is_never_a_match(gpv_mod, order, method):
+    """Saturated areas and warps past each corner (every sample reads the
+    corner's value): the target's spread is its own rounding, not what two
+    large sums about f's mean leave of each other."""
+    f = speckle()
+    sat = f.copy()
+    sat[:, 150:] = 255.0
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    for g, shifts in ((sat, [(100.0, 0.0), (110.3, 5.2), (120.0, -7.5)]),
+                      (f, [(-400.0, -400.0), (400.0, -400.0), (-400.0, 400.0), (400.0, 400.0)])):
+        G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=True)
+        d = desc(gpv_mod, shifts, order)
+        for its in (1, 5) if method == "icgn" else (1,):  # (FAGN's second warp may be anywhere)
+            got, hist = gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64, method=method, max_iterations=its,
+                                            history=True)
+            assert not got["quality_ok"].any()
+            # correlations with rounding noise are of the size n^-1/2 = 0.03
+            for z in (got["c_zncc"], hist[:, :, 1]):
+                assert np.all(np.isnan(z) | (np.abs(z) < 0.5)), (z, got["status"])
+
+
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_zero_target_ends_at_the_first_iteration(gpv_mod, order):
+    """On zeros the spread is exactly 0 whatever f's mean: the step is NaN."""
+    f = speckle()
+    g = f.copy()
+    g[:, 100:] = 0.0
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=True)
+    got, hist = gpv_mod.solve_batch(F, G, desc(gpv_mod, [(100.0, 0.0), (110.3, 5.2), (120.0, -7.5)], order),
+                                    precision=gpv_mod.PREC_FP64, max_iterations=5, history=True)
+    assert np.all(got["status"] == (5 if order == 0 else 4)) and np.all(got["iterations"] == (1 if order == 0 else 0))
+    assert np.isnan(hist[:, 0]).all() == (order == 0) and np.all(hist[:, 1:] == 0.0)
+
+
+@pytest.mark.parametrize("method", ["icgn", "fagn"])
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_target_of_another_level_costs_no_digits(oracle, gpv_mod, order, method):
+    """A target 1e5 of its contrasts away from f_m, one iteration (the level of
+    the next ones is the target's own): 1e-9 px and 1e-10 in ZNCC as elsewhere;
+    one sum about f_m leaves 1e-6 and 1e-6."""
+    a = (speckle() - 120.0) / 40.0
+    f, g = a + 5.0, np.roll(a, (2, 1), (0, 1)) + 1e5
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=True)
+    p0 = np.zeros((3, 12))
+    p0[:, 0], p0[:, 1] = 1.1, 1.9
+    d = gpv_mod.make_desc([[120.3, 140.6], [150.0, 150.0], [170.2, 133.3]], 20, order, p0)
+    kw = dict(max_iterations=1, history=True, method=method)
+    ref, rh = oracle.solve_batch(oracle.get_c(f, BORDER), oracle.get_c(g, BORDER), f.shape, BORDER, d, **kw)
+    got, gh = gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64, **kw)
+    assert np.array_equal(got["status"], ref["status"])
+    assert np.abs(got["p"][:, :2] - ref["p"][:, :2]).max() < 1e-9
+    assert np.abs(got["c_zncc"] - ref["c_zncc"]).max() < 1e-10
+    assert np.abs(gh[:, 0, 1:] - rh[:, 0, 1:]).max() < 2e-10
