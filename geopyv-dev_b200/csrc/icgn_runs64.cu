@@ -135,6 +135,21 @@ __device__ __forceinline__ double dot6(const double (&c)[6], const double (&b)[6
     return fma(c[4], b[4], fma(c[2], b[2], c[0] * b[0])) + fma(c[5], b[5], fma(c[3], b[3], c[1] * b[1]));
 }
 
+// split_clamped for the warped positions, which may lie past the range of an int:
+// base (whole) and floor(loc) are added in FP64.
+__device__ __forceinline__ void split_far(double base, double loc, int n, int &i, double &t) {
+    const double fl = floor(loc), at = base + fl;
+    t = loc - fl;
+    i = (int)at;  // a NaN gives 0, and t is NaN
+    if (at < 0.0) {
+        i = 0;
+        t = 0.0;
+    } else if (at > (double)(n - 1)) {
+        i = n - 1;
+        t = 1.0 - 1e-9;
+    }
+}
+
 // A record's parts, read once per sweep: not kept in L1.
 __device__ __forceinline__ double2 ld_pair(const double2 *p) {
     double2 v;
@@ -470,7 +485,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         const double X0 = cx + sm.p[0], Y0 = cy + sm.p[1];
         const double bxd = floor(X0), byd = floor(Y0);
         const int wbx = (int)bxd, wby = (int)byd;
-        const double ox = X0 - bxd, oy = Y0 - byd;
+        const double ox = X0 == bxd ? 0.0 : X0 - bxd, oy = Y0 == byd ? 0.0 : Y0 - byd;  // (0 at an infinity too)
         double ux = 0., uy = 0., vx = 0., vy = 0., uxx = 0., uxy = 0., uyy = 0., vxx = 0., vxy = 0., vyy = 0.;
         if (ORDER >= 1) { ux = sm.p[2 % M]; vx = sm.p[3 % M]; uy = sm.p[4 % M]; vy = sm.p[5 % M]; }
         if (ORDER == 2) {
@@ -582,8 +597,8 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     const double Lx = fma(fma(uyy, dyf, Bx), dyf, Ax), Ly = fma(fma(vyy, dyf, By), dyf, Ay);
                     int ix, iy;
                     double tx, ty;
-                    split_clamped(wbx + dx, Lx, A.w, ix, tx);
-                    split_clamped(wby + dy0 + j, Ly, A.h, iy, ty);
+                    split_far(bxd + dxf, Lx, A.w, ix, tx);
+                    split_far(byd + dyf, Ly, A.h, iy, ty);
                     double a[6], b[6], da[6], db[6], g, hx = 0.0, hy = 0.0;
                     basis(ty, a); basis(tx, b);
                     if constexpr (FAGN) { dbasis(ty, da); dbasis(tx, db); }
@@ -838,7 +853,6 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         const double *pp = sm.pprev;
         const double X0 = cx + pp[0], Y0 = cy + pp[1];
         const double bxd = floor(X0), byd = floor(Y0);
-        const int wbx = (int)bxd, wby = (int)byd;
         // this thread's template pixels; the first walk (FIRST) samples g again where the solve kept none
         auto each = [&](auto first, auto fn) {
 #pragma unroll 1
@@ -852,7 +866,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     const int sl = j * T + t;
                     const double dx = dxi, dy = dy0 + j;
                     if constexpr (!FAGN && decltype(first)::value) {
-                        double lx = X0 - bxd, ly = Y0 - byd;
+                        double lx = X0 == bxd ? 0.0 : X0 - bxd, ly = Y0 == byd ? 0.0 : Y0 - byd;
                         if (ORDER >= 1) {
                             lx += pp[2 % M] * dx + pp[4 % M] * dy;
                             ly += pp[3 % M] * dx + pp[5 % M] * dy;
@@ -863,8 +877,8 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                         }
                         int ix, iy;
                         double tx, ty;
-                        split_clamped(wbx + dxi, lx, A.w, ix, tx);
-                        split_clamped(wby + dy0 + j, ly, A.h, iy, ty);
+                        split_far(bxd + dx, lx, A.w, ix, tx);
+                        split_far(byd + dy, ly, A.h, iy, ty);
                         double a[6], b[6];
                         basis(ty, a);
                         basis(tx, b);

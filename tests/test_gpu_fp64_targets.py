@@ -109,3 +109,38 @@ def test_target_of_another_level_costs_no_digits(oracle, gpv_mod, order, method)
     assert np.abs(got["p"][:, :2] - ref["p"][:, :2]).max() < 1e-9
     assert np.abs(got["c_zncc"] - ref["c_zncc"]).max() < 1e-10
     assert np.abs(gh[:, 0, 1:] - rh[:, 0, 1:]).max() < 2e-10
+
+
+@pytest.mark.parametrize("method", ["icgn", "fagn"])
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_warps_past_the_range_of_an_int_read_the_same_edge(gpv_mod, order, method):
+    """Every sample of a warp past an edge reads that edge, however far it is
+    (src/image.rs:129-132): 3e9 px and an infinity give the sums of 4e4 px."""
+    f = speckle()
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=np.roll(f, (2, 1), (0, 1)), border=BORDER, keep_f64=True)
+    way = np.array([(1, 0), (-1, 0), (0, 1), (0, -1)], float)
+    res = []
+    for far in (4e4, 3e9, np.inf):
+        shifts = np.where(way == 0.0, 0.25, np.copysign(far, way))
+        res.append(gpv_mod.solve_batch(F, G, desc(gpv_mod, shifts, order), precision=gpv_mod.PREC_FP64, method=method,
+                                       max_iterations=1))
+        assert np.all(res[-1]["c_zncc"] != 0.0)  # a row or a column of the image is not without contrast
+    for r in res[1:]:
+        for k in ("c_zncc", "c_znssd", "status", "iterations"):
+            assert np.array_equal(r[k], res[0][k]), k
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_strains_past_the_range_of_an_int_read_both_edges(gpv_mod, order):
+    f = speckle()
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=np.roll(f, (2, 1), (0, 1)), border=BORDER, keep_f64=True)
+    res = []
+    for ux in (1e5, 1e9, 1e12):
+        d = desc(gpv_mod, [(0.3, 0.2), (0.3, 0.2)], order)
+        d["p0"][0, 2], d["p0"][1, 5] = ux, -ux
+        res.append(gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64, max_iterations=1))
+        assert np.all(res[-1]["c_zncc"] != 0.0)
+    for r in res[1:]:
+        assert np.array_equal(r["c_zncc"], res[0]["c_zncc"]) and np.array_equal(r["status"], res[0]["status"])
