@@ -201,8 +201,49 @@ __device__ __noinline__ bool compose2_any(const double *p, const double *d, doub
     return compose2(p, d, out, ws);
 }
 
+// The setup's sums about f's mean, by one warp, from the records: for a level
+// (the coefficient under the centre) that is far from the subset's values against
+// their contrast, as at a hot pixel that the mask leaves out.  tot[1], tot[2] and
+// tot[4 + j] become sum (f - m), sum (f - m)^2 and sum SDI_j (f - m).
+template <int ORDER, bool FAGN>
+__device__ __noinline__ void sums_about_mean(const double2 *RG, const double *RF, const int *RVM, const int2 *tasks, int T,
+                                             double m, double *tot, int lane) {
+    constexpr int M = Ord<ORDER>::M, N = FAGN ? 2 : 2 + M;
+    double s[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) s[q] = 0.0;
+#pragma unroll 1
+    for (int t = lane; t < T; t += 32) {
+        int dx, dy0;
+        unpack_task(tasks[t], dx, dy0);
+        const int vm = RVM[t];
+#pragma unroll 1
+        for (int j = 0; j < kK; j++) {
+            if (!((vm >> j) & 1)) continue;
+            const double a = RF[j * T + t] - m;
+            s[0] += a;
+            s[1] = fma(a, a, s[1]);
+            if constexpr (!FAGN) {
+                const double2 g = RG[j * T + t];
+#pragma unroll
+                for (int mu = 0; mu < M / 2; mu++) {
+                    const double w = mu_val<double>(mu, dx, dy0 + j) * a;
+                    s[2 + 2 * mu] = fma(g.x, w, s[2 + 2 * mu]);
+                    s[3 + 2 * mu] = fma(g.y, w, s[3 + 2 * mu]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        const double v = warp_sum(s[q]);
+        if (lane == 0) tot[q < 2 ? 1 + q : 2 + q] = v;
+    }
+    __syncwarp();
+}
+
 // One solve.  scratch (doubles, nslot slots per array, slot j * T + t for
-// pixel j of run t): the gradient pair, f - s (s the subset's level), g; for
+// pixel j of run t): the gradient pair, f, g; for
 // FAGN the target's gradient pair too; then one word of pixel bits per run.
 template <int ORDER, int NT, bool FAGN, typename C, bool ETA>
 __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, double *base, double *win,
@@ -268,7 +309,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         const double fs = v ? f - shift : 0.0;
         if (!v) gx = gy = 0.0;
         RG[sl] = make_double2(gx, gy);
-        RF[sl] = fs;
+        RF[sl] = v ? f : 0.0;  // as it is: f - s would lose digits at a far s
         if (!v) return;
         acc[0] += 1.0;
         acc[1] += fs;
@@ -398,9 +439,15 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         }
         __syncwarp();
         const int n = (int)(sm.tot[0] + 0.5);
-        const double dn = (double)n, ms = sm.tot[1] / (n > 0 ? dn : 1.0);
-        const double fm = shift + ms;
-        const double saa = fmax(sm.tot[2] - ms * sm.tot[1], 0.0);
+        const double dn = (double)n;
+        double ms = sm.tot[1] / (n > 0 ? dn : 1.0);  // mean of f - s
+        double fm = shift + ms;
+        if (n > 0 && !(sm.tot[2] - ms * sm.tot[1] > kLevelDigits * sm.tot[2])) {
+            sums_about_mean<ORDER, FAGN>(RG, RF, RVM, tasks, T, fm, sm.tot, lane);
+            ms = sm.tot[1] / dn;
+            fm += ms;
+        }
+        const double dif = sm.tot[2] - ms * sm.tot[1], saa = dif < 0.0 ? 0.0 : dif;
         int st = GPV_OK;
         if (n == 0) st = GPV_EMPTY_MASK;
         else if (!(sqrt(saa / dn) > 1e-6 * fmax(1.0, fabs(fm)))) st = GPV_FEATURELESS;
@@ -425,7 +472,6 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             sm.misc[5] = fm;
             sm.misc[6] = saa;
             sm.misc[7] = sm.tot[3];
-            sm.misc[8] = ms;
             sm.n_valid = n;
         }
     } else {
@@ -440,7 +486,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
     }
     __syncthreads();
     const int st0 = sm.flag[0], n = sm.n_valid;
-    const double dn = (double)n, fm = sm.misc[5], saa = sm.misc[6], sssig = sm.misc[7], fms = sm.misc[8];
+    const double dn = (double)n, fm = sm.misc[5], saa = sm.misc[6], sssig = sm.misc[7];
     const double df = sqrt(saa);
     if (st0 != GPV_OK) {
         if (tid == 0) {
@@ -511,7 +557,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             const double Ax = fma(fma(uxx, dxf, ux), dxf, ox), Ay = fma(fma(vxx, dxf, vx), dxf, oy);
             const double Bx = fma(uxy, dxf, uy), By = fma(vxy, dxf, vy);
             double m0x = 0.0, m0y = 0.0, m1x = 0.0, m1y = 0.0, m2x = 0.0, m2y = 0.0;
-            auto take = [&](int j, double dyf, double g, double hx, double hy, double2 gf, double fs) {
+            auto take = [&](int j, double dyf, double g, double hx, double hy, double2 gf, double f) {
                 const int sl = j * T + t;
                 const bool in = (vm >> j) & 1u;
                 if constexpr (FAGN) {
@@ -521,7 +567,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     sb += b;
                     sbb = fma(b, b, sbb);
                 } else {
-                    const double a = in ? fs - fms : 0.0, b = in ? g - cg : 0.0;
+                    const double a = in ? f - fm : 0.0, b = in ? g - cg : 0.0;
                     const double e = fma(-rho, b, a);
                     sb += b;
                     sbb = fma(b, b, sbb);
@@ -543,10 +589,10 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 for (int j = 0; j < kK; j++) {
                     const double dyf = dy0 + j;
                     double2 gf = make_double2(0.0, 0.0);  // from L2: asked for at the sample's start
-                    double fs = 0.0;
+                    double f = 0.0;
                     if constexpr (!FAGN) {
                         gf = ld_pair(RG + j * T + t);
-                        fs = ld_one(RF + j * T + t);
+                        f = ld_one(RF + j * T + t);
                     }
                     double Lx = Ax, Ly = Ay;
                     if (ORDER == 1) { Lx = fma(Bx, dyf, Lx); Ly = fma(By, dyf, Ly); }
@@ -588,7 +634,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                         for (int rr = 0; rr < 6; rr++) sr[rr] = dot6(Rg[(j + rr) % 6], w);
                         hx = dot6(sr, aw);
                     }
-                    take(j, dyf, g, hx, hy, gf, fs);
+                    take(j, dyf, g, hx, hy, gf, f);
                 }
             } else {
 #pragma unroll 1
@@ -666,7 +712,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     // offsets from the warped centre
                     const double X = fma(fma(uyy, dyf, Bx), dyf, Ex), Y = fma(fma(vyy, dyf, By), dyf, Ey);
                     const double2 h = RH[sl];
-                    const double a = RF[sl] - fms, b = RT[sl] - gm;
+                    const double a = RF[sl] - fm, b = RT[sl] - gm;
                     const double z = fma(a, inv_df, -(b * inv_dg));
                     ac[M] = fma(z, z, ac[M]);
                     const double res = fma(a, ratio, -b);
@@ -885,7 +931,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                         RT[sl] = contract<double>(GC + (int64_t)(iy + B - 2) * cp + (ix + B - 2), cp, a, b);
                     }
                     const double2 q = RG[sl];
-                    fn(RF[sl] - fms, q.x, q.y, RT[sl] - gm_last, dx, dy);
+                    fn(RF[sl] - fm, q.x, q.y, RT[sl] - gm_last, dx, dy);
                 }
             }
         };

@@ -144,3 +144,28 @@ def test_strains_past_the_range_of_an_int_read_both_edges(gpv_mod, order):
         assert np.all(res[-1]["c_zncc"] != 0.0)
     for r in res[1:]:
         assert np.array_equal(r["c_zncc"], res[0]["c_zncc"]) and np.array_equal(r["status"], res[0]["status"])
+
+
+@pytest.mark.parametrize("method", ["icgn", "fagn"])
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_masked_hot_centre_costs_no_digits(oracle, gpv_mod, order, method):
+    """A pixel of 1e8 in f that the mask leaves out with 24 px around it: f_m,
+    delta_f and the solve are those of the remaining pixels, 1e-9 px and 1e-10
+    in ZNCC of the oracle's as elsewhere, from the same coefficients (another
+    prefilter's rounding of such a pixel is 1e-8 near it)."""
+    f = speckle()
+    g = np.roll(f, (2, 1), (0, 1))
+    f[140, 120] = 1e8
+    mask = np.ones(f.shape, np.uint8)
+    mask[116:165, 96:145] = 0
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=True)
+    d = desc(gpv_mod, [(1.1, 1.9)], order, radius=45, at=(120.0, 140.0))
+    kw = dict(max_iterations=3, history=True, method=method)
+    got, gh = gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64, global_mask=gpv_mod.Mask("global", binary=mask), **kw)
+    ref, rh = oracle.solve_batch(F.coef(f64=True), G.coef(f64=True), f.shape, BORDER, d, mask=mask, **kw)
+    assert got["n_px"][0] == ref["n_px"][0] > 3000 and np.array_equal(got["status"], ref["status"])
+    assert abs(got["delta_f"][0] / ref["delta_f"][0] - 1) < 1e-12 and abs(got["f_m"][0] - ref["f_m"][0]) < 1e-10
+    assert np.abs(got["p"][:, :2] - ref["p"][:, :2]).max() < 1e-9
+    assert np.abs(got["c_zncc"] - ref["c_zncc"]).max() < 1e-10
+    assert np.abs(gh[0, :, 1:] - rh[0, :, 1:]).max() < 2e-10
