@@ -123,9 +123,10 @@ __device__ __forceinline__ int4 run_extent(const double *p, double cx, double cy
 // then solves L x = e_c for column c of L^-1, in the same shifted form.
 // Lw: M * M + 16 scratch (columns of L); Li: L^-1, row-major, zeros above the
 // diagonal; linv: M scratch; dsc: 1 / sqrt(H_jj).  False (warp-uniform) when
-// a pivot is not positive or not finite: a singular Hessian.
+// a pivot is not above min_piv (the scaled diagonal is 1) or not finite: a singular Hessian.
 template <int ORDER>
-__device__ __forceinline__ bool hess_factor(const double *mom, double *Lw, double *Li, double *linv, double *dsc, int lane) {
+__device__ __forceinline__ bool hess_factor(const double *mom, double *Lw, double *Li, double *linv, double *dsc, int lane,
+                                            double min_piv = 0.0) {
     using O = Ord<ORDER>;
     constexpr int M = O::M;
     constexpr unsigned kAll = 0xffffffffu;
@@ -147,7 +148,7 @@ __device__ __forceinline__ bool hess_factor(const double *mom, double *Lw, doubl
 #pragma unroll 1
     for (int k = 0; k < M; k++) {
         const double piv = __shfl_sync(kAll, h[0], k);
-        if (!(piv > 0.0) || !isfinite(piv)) return false;  // uniform: every lane has lane k's value
+        if (!(piv > min_piv) || !isfinite(piv)) return false;  // uniform: every lane has lane k's value
         const double rk = rsqrt(piv);
         const double lik = li > k ? h[0] * rk : (li == k ? piv * rk : 0.0);
         if (lane < M) Lw[k * M + lane] = lik;

@@ -32,9 +32,10 @@
 //  * FAGN takes two sweeps: target value and gradient at the warped positions
 //    (kept per pixel), then the Hessian's moments and the residual gradient
 //    about the warped centre.
-//  * The Hessian is factored by one warp (hess_factor); a matrix that the
-//    factor rejects goes to the pivoted elimination (gj_inverse), so only what
-//    that rejects is singular.  Second-order composition eliminates without
+//  * The Hessian is factored by one warp (hess_factor); a matrix with a scaled
+//    pivot of kMinPivot or less (rank-deficient to rounding, where a residue would pass
+//    for a pivot, or nearly so) goes to the pivoted elimination (gj_inverse),
+//    so only what that rejects is singular.  Second-order composition eliminates without
 //    pivoting while the pivots stay near 1, else with pivoting.
 // Measured against one sweep-per-sum block of 256 threads with taps through L1
 // (icgn_fp64, fagn_kernel; 254 registers, 8 warps per SM, FP64 pipe 14 % and
@@ -55,6 +56,7 @@ constexpr int kK = kRunK;
 // The sums about a level are used while they leave the spread all but two of
 // its digits (a target ten times its contrast away from the level), and the
 // residual's sum while the scale of the iteration before is within 32 times the new one.
+constexpr double kMinPivot = 1e-10;  // about the square root of a rounding's share of the unit diagonal, and less
 constexpr double kLevelDigits = 0.01, kScaleDigits = 32.0 * 32.0;
 
 template <int NW>
@@ -238,6 +240,51 @@ __device__ __noinline__ void sums_about_mean(const double2 *RG, const double *RF
     for (int q = 0; q < N; q++) {
         const double v = warp_sum(s[q]);
         if (lane == 0) tot[q < 2 ? 1 + q : 2 + q] = v;
+    }
+    __syncwarp();
+}
+
+// The gradient moments again, by one warp, each pixel's gradient product times
+// the whole monomial: where offsets depend on one another (a mask of one line)
+// the Hessian's rows then do so to the last bit, as the elimination's test for an
+// exact zero needs; the setup's powers of dy per run round in between.
+template <int ORDER>
+__device__ __noinline__ void moments_of_monomials(const double2 *RG, const int *RVM, const int2 *tasks, int T, double *mom,
+                                                  int lane) {
+    constexpr int NMOM = Ord<ORDER>::NMOM, NB = 2 * Ord<ORDER>::DEG + 1;
+#pragma unroll 1
+    for (int pr = 0; pr < 3; pr++) {
+        double s[NMOM];
+#pragma unroll
+        for (int q = 0; q < NMOM; q++) s[q] = 0.0;
+#pragma unroll 1
+        for (int t = lane; t < T; t += 32) {
+            int dx, dy0;
+            unpack_task(tasks[t], dx, dy0);
+            const int vm = RVM[t];
+#pragma unroll 1
+            for (int j = 0; j < kK; j++) {
+                if (!((vm >> j) & 1)) continue;
+                const double2 g = RG[j * T + t];
+                const double gg = (pr == 2 ? g.y : g.x) * (pr == 0 ? g.x : g.y);
+                double xp = 1.0;
+#pragma unroll
+                for (int a = 0; a < NB; a++) {
+                    double mono = xp;
+#pragma unroll
+                    for (int b = 0; a + b < NB; b++) {
+                        s[mom_idx(a, b)] = fma(gg, mono, s[mom_idx(a, b)]);
+                        mono *= dy0 + j;
+                    }
+                    xp *= dx;
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NMOM; q++) {
+            const double v = warp_sum(s[q]);
+            if (lane == 0) mom[pr * NMOM + q] = v;
+        }
     }
     __syncwarp();
 }
@@ -458,8 +505,9 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
             }
             for (int q = lane; q < 3 * NMOM; q += 32) sm.mom[q] = sm.tot[NVA + q];
             __syncwarp();
-            const bool ok = hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane);
+            const bool ok = hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane, kMinPivot);
             if (!ok) {
+                moments_of_monomials<ORDER>(RG, RVM, tasks, T, sm.mom, lane);
                 assemble_hessian<ORDER>(sm.mom, sm.L, lane);
                 int g = 0;
                 if (lane == 0) g = gj_inverse<M>(sm.L, sm.Hi);
@@ -763,7 +811,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 __syncwarp();
                 znssd = sm.tot[M];
                 // dp = H^-1 grad by the factor's inverse: D L^-T (L^-1 (D grad))
-                if (hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane)) {
+                if (hess_factor<ORDER>(sm.mom, sm.Hi, sm.L, sm.linv, sm.dsc, lane, kMinPivot)) {
                     double y = 0.0;
                     if (lane < M) {
 #pragma unroll
