@@ -18,14 +18,16 @@
 //  * ICGN takes one sweep per iteration: about a level c (the target's mean of
 //    the iteration before, f's mean at first) it sums b = g - c, b^2, a b
 //    (a = f - f_m), e^2 (e = a - rho b, rho = delta_f / delta_g of the
-//    iteration before) and SDI_j b.  With t = delta_f / delta_g,
+//    iteration before) and SDI_j e.  With t = delta_f / delta_g,
 //    k = t - rho and d the mean of b,
 //        residual r = a - t (b - d) = e - k b + t d
-//        grad_j   = sum SDI_j a - t (sum SDI_j b - d sum SDI_j)
+//        grad_j   = sum SDI_j e - k sum SDI_j b + t d sum SDI_j,
+//                   sum SDI_j b = (sum SDI_j a - sum SDI_j e) / rho
 //        ZNSSD    = sum r^2 / delta_f^2,
 //    where sum r^2 follows from sum e^2 and small corrections (k and d go to
-//    zero as the solve converges), so ZNSSD keeps the relative accuracy of the
-//    direct sum.  That costs digits where the target's level is far from c against
+//    zero as the solve converges), so ZNSSD and the gradient keep the relative
+//    accuracy of the direct sums over the residual (a difference of sums of
+//    SDI_j a and SDI_j b cost an ill-conditioned subset 1e-5 px).  That costs digits where the target's level is far from c against
 //    its contrast (a first iteration on a target of another brightness, or
 //    one without contrast), or rho far above t: there three more sweeps take the
 //    mean, the spread about it and the direct sums.
@@ -621,7 +623,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     sbb = fma(b, b, sbb);
                     sab = fma(a, b, sab);
                     see = fma(e, e, see);
-                    const double gxb = gf.x * b, gyb = gf.y * b;
+                    const double gxb = gf.x * e, gyb = gf.y * e;
                     m0x += gxb;
                     m0y += gyb;
                     if (ORDER >= 1) { m1x = fma(gxb, dyf, m1x); m1y = fma(gyb, dyf, m1y); }
@@ -858,8 +860,11 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 const double srr = sweep == 3 ? tee  // rho is t
                                               : tee + k * (k * tbb - 2.0 * (tab - rho * tbb)) - 2.0 * td * (rho * tb + k * tb) + dn * td * td;
                 znssd = (srr < 0.0 ? 0.0 : srr) / saa;  // a NaN (delta_g = 0) stays one
-                const double bj = __shfl_down_sync(0xffffffffu, tl, 4);
-                if (lane < M) sm.grad[lane] = sm.A[lane] - t_fg * (bj - gmt * sm.S[lane]);
+                const double ej = __shfl_down_sync(0xffffffffu, tl, 4);
+                if (lane < M) {
+                    const double corr = k == 0.0 ? 0.0 : k * ((sm.A[lane] - ej) / rho);
+                    sm.grad[lane] = ej - corr + td * sm.S[lane];
+                }
                 __syncwarp();
                 if (lane < M) {
                     double a0 = 0.0, a1 = 0.0;

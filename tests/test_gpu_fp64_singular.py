@@ -50,7 +50,7 @@ def test_pixels_on_one_line_are_singular(oracle, gpv_mod, order, line):
         assert np.all(fagn["status"] == 3)
 
 
-@pytest.mark.parametrize("order,method", [(0, "fagn"), (1, "icgn"), (1, "fagn")])
+@pytest.mark.parametrize("order,method", [(0, "icgn"), (0, "fagn"), (1, "icgn"), (1, "fagn")])
 def test_nearly_singular_matrices_are_solved(oracle, gpv_mod, order, method):
     """f = a(x + y) + 1e-6 b(x - y), moved by whole pixels: the scaled Hessian's
     last pivots are about 1e-12.  Order 0 finds the shift: along x + y as sharply as ever
