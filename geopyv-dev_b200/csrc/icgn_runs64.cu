@@ -831,6 +831,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     int g = 0;
                     if (lane == 0) g = gj_inverse<M>(sm.L, sm.Hi);
                     ok = __shfl_sync(0xffffffffu, g, 0) != 0;
+                    __syncwarp();  // lane 0's inverse is read below (a shuffle orders no memory)
                     if (ok && lane < M)
                         for (int k = 0; k < M; k++) dpj = fma(sm.Hi[lane * M + k], sm.tot[k], dpj);
                 }

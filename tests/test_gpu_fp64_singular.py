@@ -86,3 +86,19 @@ def test_nearly_singular_matrices_are_solved(oracle, gpv_mod, order, method):
     for r in (ref, one):
         e = r["p"][:, :2] - [1.0, -2.0]
         assert np.abs(e.sum(1)).max() < 1e-9 and np.abs(e[:, 0] - e[:, 1]).max() < 1e-6
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_fagn_elimination_is_read_after_it_is_written(gpv_mod, order):
+    """FAGN's step by the elimination's inverse, which one lane writes and the
+    others read: 128 copies of subsets that the factor rejects, the same bytes."""
+    f, g, mask, xy = _case(gpv_mod, "slope")
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=True)
+    p0 = np.zeros((len(xy), 12))
+    p0[:, 0], p0[:, 1] = 1.1, 1.9
+    d = np.repeat(gpv_mod.make_desc(xy, 20, order, p0), 128)
+    got = gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64, global_mask=gpv_mod.Mask("global", binary=mask),
+                              max_iterations=1, method="fagn")
+    for k in range(len(xy)):
+        assert len(set(r.tobytes() for r in got[128 * k:128 * k + 128])) == 1, k
