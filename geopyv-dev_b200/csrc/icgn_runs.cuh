@@ -5,11 +5,11 @@
 #include <type_traits>
 
 #include "icgn_common.cuh"
+#include "run_window.h"
 
 namespace gpv {
 namespace {
 
-constexpr int kRunMargin = 2;  // pixels a window reaches past the warped square
 constexpr int kRunK = 4;       // template pixels per run
 
 struct RunArgs {
@@ -41,35 +41,6 @@ inline void run_tables(const gpv_context *ctx, RunArgs &R) {
     R.task_off = t;
     R.task_n = t + R1;
     R.tasks = reinterpret_cast<const int2 *>(t + 2 * R1);
-}
-
-// Window row pitch in elements: a multiple of 4 (16-byte rows for cp.async)
-// that is not a multiple of BANKS, the elements one row of shared-memory banks
-// holds (32 floats, 16 doubles), so two bands' rows read by one warp start on
-// different banks.  Lanes of a warp read consecutive columns of one row.
-template <int BANKS>
-__host__ __device__ __forceinline__ int run_pitch(int ww) {
-    const int p = (ww + 3) & ~3;
-    return (p & (BANKS - 1)) ? p : p + 4;
-}
-
-// A window covering pixel indices [xlo, xhi] x [ylo, yhi] (clamped to the
-// image) plus the taps and kRunMargin; false if it does not fit in cap
-// elements (the margin is dropped when the window with it does not fit).
-template <int BANKS>
-__device__ __forceinline__ bool run_plan(int xlo, int xhi, int ylo, int yhi, int border, int cap, int &r0, int &c0,
-                                         int &wh, int &ww, int &pitch) {
-    for (int m = kRunMargin; m >= 0; m -= kRunMargin) {
-        const int clo = xlo + border - 2 - m, chi = xhi + border + 3 + m;
-        c0 = clo >= 0 ? (clo & ~3) : -(((-clo) + 3) & ~3);
-        ww = ((chi + 1 - c0) + 3) & ~3;
-        pitch = run_pitch<BANKS>(ww);
-        r0 = ylo + border - 2 - m;
-        wh = yhi + border + 3 + m + 1 - r0;
-        if (pitch * wh <= cap) return true;
-        if (m == 0) break;
-    }
-    return false;
 }
 
 template <class S>

@@ -122,7 +122,7 @@ __device__ __forceinline__ bool plan_window(int xlo, int xhi, int ylo, int yhi, 
         ww = window_pitch(((chi + 1 - c0) + 3) & ~3, layout);
         r0 = ylo + border - 2 - m;
         wh = yhi + border + 3 + m + 1 - r0;
-        if (ww * wh <= cap) return true;
+        if ((int64_t)ww * wh <= cap) return true;
         if (m == 0) break;
     }
     return false;
