@@ -1175,54 +1175,6 @@ const void *run_kernel_nt(int order, RunForm form, bool eta) {
 // Host side: run tables, sizes and launches (called by the batched launcher).
 // ---------------------------------------------------------------------------
 
-// Run tables for radii 1..max_radius: per run {dx (low 16 bits) | dy0 (high
-// 16 bits), circle bits}, bands of kRunK rows from dy = -r, the last band
-// moved up to end at dy = r (its rows already in the band above masked off);
-// columns [-w, w] with w the widest circle row of the band.
-int ensure_run_tables(gpv_context *ctx, int max_radius) {
-    if (max_radius <= ctx->run_table_radius) return GPV_SUCCESS;
-    const int R1 = max_radius + 1;
-    std::vector<int32_t> tab;  // pairs
-    std::vector<int32_t> off(R1, 0), cnt(R1, 0);
-    for (int r = 1; r <= max_radius; r++) {
-        off[r] = (int32_t)(tab.size() / 2);
-        int n = 0;
-        for (int b0 = -r; b0 <= r; b0 += kRunK) {
-            const int dy0 = (2 * r + 1 >= kRunK) ? std::min(b0, r - kRunK + 1) : -r;
-            int w = -1;
-            for (int j = 0; j < kRunK; j++) {
-                const int y = dy0 + j;
-                if (y < b0 || y > r) continue;
-                // the row's exact integer half-width, then the band's widest
-                int h = (int)std::floor(std::sqrt((double)(r * r - y * y)));
-                while ((h + 1) * (h + 1) + y * y <= r * r) h++;
-                while (h > 0 && h * h + y * y > r * r) h--;
-                w = std::max(w, h);
-            }
-            for (int dx = -w; dx <= w; dx++) {
-                uint32_t bits = 0;
-                for (int j = 0; j < kRunK; j++) {
-                    const int y = dy0 + j;
-                    if (y >= b0 && y <= r && dx * dx + y * y <= r * r) bits |= 1u << j;
-                }
-                tab.push_back((int32_t)((uint32_t)(dx & 0xffff) | ((uint32_t)dy0 << 16)));
-                tab.push_back((int32_t)bits);
-                n++;
-            }
-        }
-        cnt[r] = n;
-    }
-    // one buffer, one copy: run offsets, run counts, runs (8-byte aligned)
-    std::vector<int32_t> all(off);
-    all.insert(all.end(), cnt.begin(), cnt.end());
-    all.insert(all.end(), tab.begin(), tab.end());
-    if (int rc = ctx->run_tab.ensure(all.size() * sizeof(int32_t))) return rc;
-    GPV_CUDA_TRY(cudaMemcpy(ctx->run_tab.ptr, all.data(), all.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    ctx->h_run_n = cnt;
-    ctx->run_table_radius = max_radius;
-    return GPV_SUCCESS;
-}
-
 // Window capacity (floats) of a launch for subsets up to radius rmax: the
 // square of half side max(rmax, kRunK - 1 - rmax) stretched by 6%, taps and
 // margins, at a pitch of whole 32-float rows.

@@ -10,8 +10,6 @@
 namespace gpv {
 namespace {
 
-constexpr int kRunK = 4;       // template pixels per run
-
 struct RunArgs {
     KArgs k;
     const int2 *tasks;        // run tables

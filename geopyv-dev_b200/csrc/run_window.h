@@ -1,5 +1,6 @@
-// run_window.h -- planning of the coefficient windows that the run-layout solves
-// stage in shared memory (host and device; no CUDA header needed).
+// run_window.h -- the run length of the run-layout solves and the planning of the
+// coefficient windows they stage in shared memory (host and device; no CUDA
+// header needed).
 #pragma once
 #include <cstdint>
 
@@ -12,6 +13,7 @@
 namespace gpv {
 namespace {
 
+constexpr int kRunK = 4;       // template pixels per run
 constexpr int kRunMargin = 2;  // pixels a window reaches past the warped square
 
 // Window row pitch in elements: a multiple of 4 (16-byte rows for cp.async)
