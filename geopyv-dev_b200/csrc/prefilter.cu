@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "internal.h"
 
@@ -85,9 +86,12 @@ Poles poles() {
 // At MT = kM32 the slow pole's taps past |m| = MT, which the lead-in of the
 // other outputs brings with it, are taken off again (the chain's state MT + 1
 // samples back, times t1): every output is the filter of 2 MT + 1 taps, to FP64
-// rounding, wherever it lies in its group.
+// rounding, wherever it lies in its group.  A sample that is not finite stays in
+// the chains to the group's end: false says that there is one, and the caller
+// takes the group's outputs again tap by tap (tap_by_tap), so that it reaches
+// |m| = MT and no farther.
 template <int MT, class X>
-__device__ __forceinline__ void exponentials(X x, const Poles &c, double (&acc)[kQ]) {
+__device__ __forceinline__ bool exponentials(X x, const Poles &c, double (&acc)[kQ]) {
     constexpr bool kCut = MT == kM32;
     constexpr int W2 = MT <= 28 ? 8 : 13;
     double p1 = 0.0, p2 = 0.0, s1 = 0.0, s2 = 0.0;
@@ -113,6 +117,20 @@ __device__ __forceinline__ void exponentials(X x, const Poles &c, double (&acc)[
             if (q < kQ) acc[q] = fma(c.b1, s1, fma(c.b2, s2, acc[q]));
         }
     }
+    return isfinite(p1) && isfinite(s1);
+}
+
+// One output tap by tap, x its sample.
+template <int MT, class S>
+__device__ __noinline__ double tap_by_tap(const S *x, int stride, double z1, double z2, double a1, double a2) {
+    double acc = (a1 + a2) * (double)x[0];
+#pragma unroll 1
+    for (int m = 1; m <= MT; m++) {
+        a1 *= z1;
+        a2 *= z2;
+        acc = fma(a1 + a2, (double)x[m * stride], fma(a1 + a2, (double)x[-m * stride], acc));
+    }
+    return acc;
 }
 
 // Both passes in one kernel.  A block owns a strip of kStrip padded columns
@@ -157,6 +175,7 @@ __global__ void __launch_bounds__(kFusedThreads, 3) prefilter_fused(const P *__r
                                                                 float *__restrict__ c32, int64_t pitch32,
                                                                 double *__restrict__ c64, int64_t pitch64) {
     using G = Fused<P, MT>;
+    constexpr bool kAny = std::is_floating_point<P>::value;  // pixels may be NaN or infinite
     extern __shared__ double smem[];
     double *ring = smem;
     P *pxs = reinterpret_cast<P *>(reinterpret_cast<unsigned char *>(smem) + G::kRingBytes);
@@ -214,10 +233,14 @@ __global__ void __launch_bounds__(kFusedThreads, 3) prefilter_fused(const P *__r
         if (rr < n) {
             const P *x = pxs + rr * G::kPxPitch + half * kQ;
             double acc[kQ];
-            exponentials<MT>([&](int sx) { return (double)x[sx]; }, poles, acc);
+            const bool fine = exponentials<MT>([&](int sx) { return (double)x[sx]; }, poles, acc);
             double *o = ring + (dst + rr) * G::kRingPitch + half * kQ;
 #pragma unroll
             for (int q = 0; q < kQ; q++) o[q] = acc[q];
+            if (kAny && !fine) {
+#pragma unroll 1
+                for (int q = 0; q < kQ; q++) o[q] = tap_by_tap<MT>(x + MT + q, 1, poles.z1, poles.z2, poles.a1, poles.a2);
+            }
         }
         __syncthreads();
     };
@@ -232,7 +255,7 @@ __global__ void __launch_bounds__(kFusedThreads, 3) prefilter_fused(const P *__r
         if (wid * kQ < n) {
             const double *x = ring + (wid * kQ) * G::kRingPitch + lane;
             double acc[kQ];
-            exponentials<MT>([&](int sx) { return x[sx * G::kRingPitch]; }, poles, acc);
+            const bool fine = exponentials<MT>([&](int sx) { return x[sx * G::kRingPitch]; }, poles, acc);
             const int64_t j = j0 + lane;
             if (j < cw) {
 #pragma unroll
@@ -241,6 +264,15 @@ __global__ void __launch_bounds__(kFusedThreads, 3) prefilter_fused(const P *__r
                         const int64_t i = i_beg + done + wid * kQ + q;
                         c32[i * pitch32 + j] = (float)acc[q];
                         if (c64) c64[i * pitch64 + j] = acc[q];
+                    }
+                }
+                if (kAny && !fine) {
+#pragma unroll 1
+                    for (int q = 0; q < kQ && wid * kQ + q < n; q++) {
+                        const int64_t i = i_beg + done + wid * kQ + q;
+                        const double v = tap_by_tap<MT>(x + (MT + q) * G::kRingPitch, G::kRingPitch, poles.z1, poles.z2, poles.a1, poles.a2);
+                        c32[i * pitch32 + j] = (float)v;
+                        if (c64) c64[i * pitch64 + j] = v;
                     }
                 }
             }

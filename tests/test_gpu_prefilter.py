@@ -151,3 +151,30 @@ def test_group_and_strip_edges_match_oracle(oracle, gpv_mod, shape, keep_f64):
     assert np.abs(im.coef().astype(np.float64) - ref).max() <= 2e-7 * scale
     if keep_f64:
         assert np.abs(im.coef(f64=True) - ref).max() <= 1e-8 * scale
+
+
+@pytest.mark.parametrize("at", [(140, 151), (5, 250), (176, 3)])
+@pytest.mark.parametrize("keep_f64", [False, True])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_a_pixel_that_is_not_finite_reaches_as_far_as_the_taps(gpv_mod, value, dtype, keep_f64, at):
+    """28 samples along each axis for FP32 coefficients, 44 for FP64 ones (wrapping
+    as the filter does), wherever the pixel lies in its group of outputs; an
+    infinity gives infinities, and the other coefficients are those of the image
+    with a 0 there, within this file's bounds."""
+    rng = np.random.default_rng(11)
+    img = rng.uniform(0, 255, (180, 260)).astype(dtype)
+    img[at] = 0
+    base = gpv_mod.Image(image_gs=img, border=20, keep_f64=keep_f64).coef(f64=keep_f64)
+    img[at] = value
+    im = gpv_mod.Image(image_gs=img, border=20, keep_f64=keep_f64)
+    got = im.coef(f64=keep_f64)
+    reach = 44 if keep_f64 else 28
+    hit = np.ones(got.shape, bool)
+    for ax in (0, 1):
+        n = got.shape[ax]
+        d = np.abs(np.arange(n) - (at[ax] + 20))
+        hit &= (np.minimum(d, n - d) <= reach).reshape((-1, 1) if ax == 0 else (1, -1))
+    assert np.array_equal(~np.isfinite(got), hit)
+    assert np.isnan(got[hit]).all() if np.isnan(value) else np.isinf(got[hit]).all()
+    assert np.abs(got - base)[~hit].max() <= (1e-8 if keep_f64 else 2e-7) * np.abs(base[~hit]).max()
