@@ -48,8 +48,8 @@
 //  * Sums.  The per-iteration sums g - f_m, its square and (f - f_m)(g - f_m)
 //    are FP32 over one run (at most K samples), then FP64 per thread and across
 //    the block in a fixed order (deterministic); the steepest-descent products
-//    and the setup's sums are FP32 per thread, then FP64.  64 threads take these
-//    in pairs of runs and in halves, as many terms as 128 threads have.
+//    and the setup's sums are FP32 per thread, then FP64.  64 threads keep
+//    the FP32 sums of 128: two apiece, one after the other.
 //  * Rigid texture (RIGID; orders 1 and 2): the grain maps sampled per pixel at
 //    setup, and a template pass per iteration with the sums of its correction G
 //    (the run's four pixels' loads together in flight); the sample loop only adds
@@ -409,11 +409,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     // under the centre: keeps the sums free of cancellation and a flat
     // subset's sums exactly zero); FP32 per thread, FP64 across the block.
     constexpr int NVA = 4 + 2 * M;
-    // 64 threads have twice the runs each: their FP32 sums are taken in halves,
-    // so that no more pixels than with 128 threads share one (the error of
-    // delta_f and of the ZNCC against 64 bits would be 1.5 to 2.5 times as large)
+    // 64 threads have twice the runs each: thread i takes the runs of threads i
+    // and i + 64 of 128 one after the other, in FP32 sums of their own joined in
+    // FP64, so that every FP32 sum is one that 128 threads have (the error of
+    // delta_f and of the ZNCC against 64 bits would be 1.2 to 1.9 times as large)
     constexpr int kHalves = NT == 64 ? 2 : 1;
-    const int t_half = kHalves == 2 ? (T + 2 * NT - 1) / (2 * NT) * NT : T;
     double carry = 0.0;
     float acc[NVA];
     float shift;
@@ -456,8 +456,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         for (int hf = 0; hf < kHalves; hf++) {
 #pragma unroll
         for (int q = 0; q < NVA; q++) acc[q] = 0.f;
-        const int t_end = kHalves == 2 ? min(T, (hf + 1) * t_half) : T;
-        for (int t = kHalves == 2 ? hf * t_half + tid : tid; t < t_end; t += NT) {
+        for (int t = hf * NT + tid; t < T; t += kHalves * NT) {
             int dx, dy0;
             unpack_task(tasks[t], dx, dy0);
             uint32_t vm = (uint32_t)tasks[t].y;
@@ -551,9 +550,12 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     // expanded by the run's powers of dx; each thread re-reads its own records
     {
         float mom[3 * NMOM];
+        double carry_m[(3 * NMOM + 31) / 32] = {};
+#pragma unroll 1
+        for (int hf = 0; hf < kHalves; hf++) {
 #pragma unroll
         for (int q = 0; q < 3 * NMOM; q++) mom[q] = 0.f;
-        for (int t = tid; t < T; t += NT) {
+        for (int t = hf * NT + tid; t < T; t += kHalves * NT) {
             int dx, dy0;
             unpack_task(tasks[t], dx, dy0);
             float V[3][NB];
@@ -589,6 +591,18 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                         mom[p * NMOM + mom_idx(a, b)] = fmaf(xp[a], V[p][b], mom[p * NMOM + mom_idx(a, b)]);
         }
         run_warp_sums<3 * NMOM, (NMOM > 1)>(mom, sm.part[wid], sm.red2[wid] + NVA, lane);
+        if constexpr (kHalves == 2) {
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 3 * NMOM; q += 32) {
+                if (q + lane < 3 * NMOM) {
+                    carry_m[q / 32] += sm.red2[wid][NVA + q + lane];
+                    sm.red2[wid][NVA + q + lane] = carry_m[q / 32];
+                }
+            }
+            __syncwarp();
+        }
+        }
     }
     if constexpr (RIGID) {
         if (rigid_on) {
@@ -791,11 +805,19 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
         double s1 = 0.0, s2 = 0.0, sfg = 0.0;
         KSum ks[3];
         float2 PB[6];
-        float2 PH[6];  // 64 threads: pairs of runs are added first (as the setup's halves)
-        bool pair = false;
+        float2 PH[6];  // 64 threads: the first of the two sums a thread takes (as at setup)
 #pragma unroll
         for (int k = 0; k < 6; k++) PB[k] = PH[k] = make_float2(0.f, 0.f);
-        for (int t = tid; t < T; t += NT) {
+#pragma unroll 1
+        for (int hf = 0; hf < kHalves; hf++) {
+        if (hf) {
+#pragma unroll
+            for (int k = 0; k < M / 2; k++) {
+                PH[k] = PB[k];
+                PB[k] = make_float2(0.f, 0.f);
+            }
+        }
+        for (int t = hf * NT + tid; t < T; t += kHalves * NT) {
             int dx, dy0;
             unpack_task(tasks[t], dx, dy0);
             const float dxf = (float)dx;
@@ -889,23 +911,8 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 s2 += (double)ac.p2;
                 sfg += (double)ac.pfg;
             }
-            if constexpr (NT == 64) {
-                acc_expand<ORDER>(ac, dxf, PH);
-                if (pair) {
-#pragma unroll
-                    for (int k = 0; k < M / 2; k++) {
-                        PB[k] = __fadd2_rn(PB[k], PH[k]);
-                        PH[k] = make_float2(0.f, 0.f);
-                    }
-                }
-                pair = !pair;
-            } else {
-                acc_expand<ORDER>(ac, dxf, PB);
-            }
+            acc_expand<ORDER>(ac, dxf, PB);
         }
-        if constexpr (NT == 64) {
-#pragma unroll
-            for (int k = 0; k < M / 2; k++) PB[k] = __fadd2_rn(PB[k], PH[k]);
         }
         // block sums: warp partials to shared memory, one barrier, then warp 0
         // adds them up and updates the warp; a second barrier publishes p
@@ -922,20 +929,29 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                 const double t = warp_sum(v[q]);
                 if (lane == q) sm.red[wid][q] = t;
             }
-            float pb[M];
+            float pb[kHalves * M];  // both sums of 64 threads, joined in FP64 below
 #pragma unroll
             for (int j = 0; j < M / 2; j++) {
                 pb[2 * j] = PB[j].x;
                 pb[2 * j + 1] = PB[j].y;
+                if constexpr (kHalves == 2) {
+                    pb[M + 2 * j] = PH[j].x;
+                    pb[M + 2 * j + 1] = PH[j].y;
+                }
             }
-            run_warp_sums<M, false>(pb, sm.part[wid], sm.red[wid] + 3, lane);
+            run_warp_sums<kHalves * M, false>(pb, sm.part[wid], kHalves == 2 ? sm.red2[wid] : sm.red[wid] + 3, lane);
         }
         __syncthreads();
         if (wid == 0) {
             double tl = 0.0;
             if (lane < KR) {
+                if (kHalves == 2 && lane >= 3) {
 #pragma unroll
-                for (int w = 0; w < NT / 32; w++) tl += sm.red[w][lane];
+                    for (int w = 0; w < NT / 32; w++) tl += sm.red2[w][lane - 3] + sm.red2[w][lane - 3 + M];
+                } else {
+#pragma unroll
+                    for (int w = 0; w < NT / 32; w++) tl += sm.red[w][lane];
+                }
             }
             const double t0 = __shfl_sync(0xffffffffu, tl, 0), t1 = __shfl_sync(0xffffffffu, tl, 1);
             const double t2 = __shfl_sync(0xffffffffu, tl, 2);
