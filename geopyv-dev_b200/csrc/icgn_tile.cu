@@ -1555,25 +1555,26 @@ int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n, boo
         const int t = atoi(v);
         return t == 256 ? 256 : (t == 64 ? 64 : 128);
     }
+    // a tuned choice holds for every batch of its class
+    const int cls = max_radius <= 20 ? 0 : (max_radius <= 40 ? 1 : 2);
+    if (ctx->tuned_threads[cls]) return ctx->tuned_threads[cls];
     // A batch that leaves every SM one subset at most is bound by one subset's
     // latency: 256 threads (first order, radius 25: 91 against 94 us for 256
     // subsets by the device call, a mesh's batches of tens 8 % shorter).  From
     // two subsets per SM on, 128 threads share the SM better (576 subsets: 96
     // against 110 us).
     if (n <= ctx->num_sms) return 256;
-    const int cls = max_radius <= 20 ? 0 : (max_radius <= 40 ? 1 : 2);
-    if (ctx->tuned_threads[cls]) return ctx->tuned_threads[cls];
     // 64 threads, eight subsets per SM: one subset's serial part (sums, update)
     // passes behind seven others' samples, while their windows still share the
-    // SM.  Times of 128 over 64 threads: first order, radius 18 1.05, 25 1.02,
-    // 28 0.97-1.02, 30 (windows over an eighth of the SM) 0.66-0.78; order 0,
-    // radius 16 1.03-1.05, 25 1.05-1.09; second order, radius 8 1.28, 12 1.14,
-    // 14 1.12 (64 threads also leave fewer lanes idle in the last round of its
-    // runs), 16 0.98, 20 0.99.  Below one and a half rounds of 1,184 subsets the
-    // last round weighs more (first order, radius 25: 1,444 subsets 0.95, 1,849
-    // 1.01).  Not with the omitted-mode diagnostic (1.03-1.05): it follows the
-    // parameters' last bits, and another split of the sums moves it by 5e-6 of
-    // its size.
+    // SM.  Times of 128 over 64 threads: order 0, radius 10 1.18, 16 1.09-1.14,
+    // 25 1.035; first order, radius 18 1.01-1.02, 25 0.99-1.00 for one batch by itself
+    // and 1.03 in a row of batches, 28 0.96 (windows over an eighth of the SM);
+    // second order, radius 8 1.20, 10 1.00, 12 1.06, 14 1.05-1.07, 16 0.97.  Below one
+    // and a half rounds of 1,184 subsets the last round weighs more (first
+    // order, radius 25: 1,849 subsets 0.986).  n is the whole batch's: the host
+    // does not know a device batch's segments, and a batch returns the same
+    // bytes by either call.  Not with the omitted-mode diagnostic (1.03-1.05),
+    // which follows the parameters' last bits.
     if (!eta && n >= 12 * (int64_t)ctx->num_sms && max_radius <= (order == 2 ? 14 : 25)) return 64;
     return max_radius > 40 ? 256 : 128;
 }
