@@ -932,7 +932,7 @@ static void tune_cache_load(gpv_context *ctx) {
         if (got >= 3 && cls >= 0 && cls < 3 && strcmp(name, prop.name) == 0 && (nt == 64 || nt == 128 || nt == 256)) {
             ctx->tuned_threads[cls] = nt;  // later lines win
             ctx->tuned_layout[cls] = (got >= 4 && layout >= 0 && layout <= 2) ? layout : -1;
-            ctx->tuned_run_k[cls] = (got == 5 && (runk == 4 || runk == 8)) ? runk : 0;
+            ctx->tuned_run_k[cls] = (got == 5 && (runk == 4 || runk == 8)) ? 4 : 0;  // runs of 8 are gone: solved in runs of 4
         }
     }
     fclose(fh);

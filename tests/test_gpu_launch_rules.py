@@ -32,3 +32,15 @@ def test_a_tuned_choice_holds_for_small_batches(gpv_mod, tmp_path, monkeypatch, 
     cache.write_text(f"{torch.cuda.get_device_name(0)}|1|{threads}|-1|4\n")
     monkeypatch.setenv("GPV_TUNE_CACHE", str(cache))
     assert solve() == want
+
+
+@pytest.mark.parametrize("line,want", [("|0|64|-1|8", 4), ("|0|64|-1|4", 4), ("|0|128|2|0", 0), ("|0|128|2", 0), ("|0|128", 0)])
+def test_cached_run_lengths_are_the_ones_solved_with(gpv_mod, tmp_path, monkeypatch, line, want):
+    """Cache lines of run length 8, which no kernel has any more, are reported as
+    what they run as."""
+    import torch
+    cache = tmp_path / "tune.txt"
+    cache.write_text(torch.cuda.get_device_name(0) + line + "\n")
+    monkeypatch.setenv("GPV_TUNE_CACHE", str(cache))
+    ctx = gpv_mod.Context(0)
+    assert (ctx.tuning()[0]["run_length"] or 0) == want
