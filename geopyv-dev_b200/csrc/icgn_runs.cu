@@ -87,7 +87,6 @@ struct RunSmem {
     double red[NW][16];
     double red2[NW][80];
     double aug[80];
-    double tot[16];
     double misc[10];
     int flag[4];
     int item;
@@ -368,7 +367,6 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
     const int re = max(r, K - 1 - r);  // half side of the square the runs cover
     const int T = R.task_n[r];
     const int2 *tasks = R.tasks + R.task_off[r];
-    const int NS = T * K;
     // per-pixel records (df/dx, df/dy, f - s, 1 in the template / 0 outside:
     // zero gradients outside) in slot j * T + t of run t; eta resamples; run bits
     float4 *REC = reinterpret_cast<float4 *>(base);

@@ -312,7 +312,6 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
     const int re = max(r, kK - 1 - r);
     const int T = R.task_n[r];
     const int2 *tasks = R.tasks + R.task_off[r];
-    const int NS = T * kK;
     double2 *RG = reinterpret_cast<double2 *>(base);
     double *RF = base + 2 * (int64_t)R.nslot, *RT = base + 3 * (int64_t)R.nslot;
     double2 *RH = reinterpret_cast<double2 *>(base + 4 * (int64_t)R.nslot);  // FAGN only

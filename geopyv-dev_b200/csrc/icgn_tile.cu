@@ -1280,11 +1280,6 @@ void tile_launch_one(int nt, bool per_subset, int order, bool rigid, int blocks,
 
 bool use_run_kernel();
 
-// Threads per block of the tiled kernel for subsets of radius r: the
-// autotuned choice when one was recorded for this radius class, else a
-// size rule (GPV_TILE_THREADS overrides).
-int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n, bool eta);
-
 // Raise a kernel's dynamic shared-memory limit to everything the device
 // allows beside its static shared memory, once per (device, kernel).  The
 // limit is a per-function attribute shared by every thread of the process:
@@ -1397,8 +1392,12 @@ int tile_launch(gpv_context *ctx, const KArgs &K, int64_t n, SolveForm form, cud
         if (!P.live) continue;
         P.rmax = std::min(kRBoundHost[c], K.max_radius);
         if (!mixed) {
-            // FP64 run layout: 3 blocks of 128 threads per SM up to radius 32 (the
-            // windows of three blocks fit), 256 threads where fewer windows fit
+            // FP64 run layout: 128 threads while two or three blocks' windows share an
+            // SM, 256 where one or two do.  Times of 128 over 256 threads (2,000
+            // subsets; orders 0, 1, 2): radius 16 0.56, 0.62, 0.67; 24 0.68, 0.72,
+            // 0.74; 32 0.76, 0.84, 0.79; 36 0.89, 0.99, 0.84; 40 0.90, 1.00, 0.86; 48
+            // 1.27, 1.53, 1.27; 60 1.36, 1.62, 1.37; FAGN radius 32 0.84, 0.79; 36 1.01,
+            // 0.99; 48 1.48, 1.49 (orders 1, 2): the line could lie at 40
             P.nt = P.rmax > 32 ? 256 : 128;
             if (int rc = ensure_run_tables(ctx, K.max_radius)) return rc;
             P.fn = run64_kernel(order, P.nt, fagn, K.f64 != nullptr, (K.flags & GPV_SOLVE_ETA) != 0);

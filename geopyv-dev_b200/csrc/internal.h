@@ -185,11 +185,11 @@ int mesh_drive(const double *nodes, int64_t n_nodes, const int64_t *elements, in
                gpv_subset_result *out, int32_t *rounds, gpv_mesh_stats *stats);
 // Colour ingest (load_grayscale + gaussian_blur_5x5): RGB8 (h, w, 3) -> u8 grey.
 int ingest_launch(const uint8_t *rgb_dev, int64_t h, int64_t w, uint8_t *grey_dev, cudaStream_t s);
-// Threads per block (batches of n subsets) / template layout (0 compact, 1
-// padded rows, 2 tiles) of the tiled solve for subsets up to max_radius:
-// GPV_TILE_THREADS / GPV_TILE_LAYOUT, else a candidate being timed, else the
-// tuned choice.
-int tile_threads_for(gpv_context *ctx, int max_radius, int64_t n);
+// Threads per block (order, batches of n subsets, with the omitted-mode
+// diagnostic) / template layout (0 compact, 1 padded rows, 2 tiles) of the
+// mixed-precision solve for subsets up to max_radius: a candidate being timed, else
+// GPV_TILE_THREADS / GPV_TILE_LAYOUT, else the tuned choice, else a rule.
+int tile_threads_for(gpv_context *ctx, int order, int max_radius, int64_t n, bool eta);
 int tile_layout_for(gpv_context *ctx, int max_radius);
 // The (order, radius class) segment of the tiled solve that holds a valid
 // subset of radius r and warp order o (0 <= q < kTileSegs); a host batch's
