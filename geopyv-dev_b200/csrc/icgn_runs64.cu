@@ -41,9 +41,9 @@
 //    pivoting while the pivots stay near 1, else with pivoting.
 // Measured against one sweep-per-sum block of 256 threads with taps through L1
 // (icgn_fp64, fagn_kernel; 254 registers, 8 warps per SM, FP64 pipe 14 % and
-// 29 % busy): 8,836 second-order subsets of radius 30 12.53 -> 2.40 ms (FP64
-// pipe 40 %), 2,401 first-order FAGN solves of radius 25 on FP32 coefficients
-// 1.27 -> 0.62 ms (47 %).
+// 29 % busy): 8,836 second-order subsets of radius 30 12.53 -> 2.28 ms (FP64
+// pipe 46 %), 2,304 first-order FAGN solves of radius 25 on FP32 coefficients
+// 1.27 -> 0.63 ms (48 %).
 // Samples that can meet the image's edge, and windows that do not fit in
 // shared memory, take a clamped per-sample path (src/image.rs:129-132).
 #include <algorithm>

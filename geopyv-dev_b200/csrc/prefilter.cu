@@ -27,7 +27,7 @@
 // and the shared-memory reads bound it (FP64 pipe 17-25 %), so a warp has the
 // loads of kAhead lines in flight and three blocks share an SM (80 registers).
 // 4096^2 u16 207 -> 125 us, 2048^2 u8 63 -> 37, 911 x 1237 f64 with FP64
-// coefficients 102 -> 26, 4096^2 f32 with FP64 coefficients 596 -> 279.  Groups of kQ outputs start at multiples of kQ
+// coefficients 102 -> 28, 4096^2 f32 with FP64 coefficients 596 -> 276.  Groups of kQ outputs start at multiples of kQ
 // of the padded line, so an output does not depend on how the rows are cut
 // into launches and blocks.  Both passes run in one kernel (prefilter_fused):
 // first along staged pixel rows, then down a ring of FP64 row-pass lines held in

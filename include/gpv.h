@@ -222,7 +222,11 @@ int gpv_mask_destroy(gpv_mask *m);
  * (src/subset.rs:836-919, :1117-1219) as called from
  * Mesh::solve_one_with_tolerance (src/mesh.rs:1025-1040) and
  * PySubset::solve_icgn (python/src/py_subset.rs:217-237).
- * Host arrays in and out; synchronous. */
+ * Host arrays in and out; synchronous.
+ * Results are the same bytes from run to run.  A mixed-precision subset's last
+ * bits depend on its batch: on the batch's size (one subset per SM or less, or
+ * twelve per SM or more, are solved with other numbers of threads, which sum in
+ * another order) and on the largest radius that is solved with it. */
 int gpv_solve_batch(gpv_context *ctx, const gpv_image *f, const gpv_image *g, const gpv_subset_desc *desc,
                     int64_t n, const gpv_solve_params *params, gpv_subset_result *out);
 /* Device arrays in and out, asynchronous on `stream` (a cudaStream_t, or
@@ -476,7 +480,7 @@ int gpv_context_tuning(gpv_context *ctx, int32_t *threads, int32_t *layouts);
 typedef struct {
     int32_t threads;            /* threads per block: 64, 128 or 256                    */
     int32_t layout;             /* tiled kernel's template layout (-1, 0, 1, 2)         */
-    int32_t run_length;         /* run-layout kernel: template pixels per run (4)       */
+    int32_t run_length;         /* run-layout kernel: template pixels per run (4; 0: not tuned) */
     int32_t subsets_per_block;  /* subsets a block solves side by side (1 or 2)         */
     int32_t staging;            /* coefficient-window buffers per subset (1 or 2)       */
     int32_t reserved;
