@@ -139,6 +139,13 @@ __device__ __forceinline__ double dot6(const double (&c)[6], const double (&b)[6
     return fma(c[4], b[4], fma(c[2], b[2], c[0] * b[0])) + fma(c[5], b[5], fma(c[3], b[3], c[1] * b[1]));
 }
 
+// One chain, in the taps' order: on equal coefficients the two chains of dot6
+// cancel a derivative's weights to exactly 0 (a saturated target would have a
+// singular FAGN Hessian), this one to its rounding as contract_grad does.
+__device__ __forceinline__ double seq6(const double (&c)[6], const double (&b)[6]) {
+    return fma(c[5], b[5], fma(c[4], b[4], fma(c[3], b[3], fma(c[2], b[2], fma(c[1], b[1], c[0] * b[0])))));
+}
+
 // split_clamped for the warped positions, which may lie past the range of an int:
 // base (whole) and floor(loc) are added in FP64.
 __device__ __forceinline__ void split_far(double base, double loc, int n, int &i, double &t) {
@@ -677,11 +684,11 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                     if constexpr (FAGN) {
                         double w[6];
                         dbasis(ty, w);
-                        hy = dot6(sr, w);
+                        hy = seq6(sr, w);
                         dbasis(tx, w);
 #pragma unroll
-                        for (int rr = 0; rr < 6; rr++) sr[rr] = dot6(Rg[(j + rr) % 6], w);
-                        hx = dot6(sr, aw);
+                        for (int rr = 0; rr < 6; rr++) sr[rr] = seq6(Rg[(j + rr) % 6], w);
+                        hx = seq6(sr, aw);
                     }
                     take(j, dyf, g, hx, hy, gf, f);
                 }
