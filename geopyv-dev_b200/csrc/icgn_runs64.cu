@@ -29,8 +29,9 @@
 //    accuracy of the direct sums over the residual (a difference of sums of
 //    SDI_j a and SDI_j b cost an ill-conditioned subset 1e-5 px).  That costs digits where the target's level is far from c against
 //    its contrast (a first iteration on a target of another brightness, or
-//    one without contrast), or rho far above t: there three more sweeps take the
-//    mean, the spread about it and the direct sums.
+//    one without contrast), rho far above t, or a Hessian near singular (few
+//    pixels: only the direct sum's rounding stays where its inverse is small):
+//    there three more sweeps take the mean, the spread about it and the direct sums.
 //  * FAGN takes two sweeps: target value and gradient at the warped positions
 //    (kept per pixel), then the Hessian's moments and the residual gradient
 //    about the warped centre.
@@ -597,7 +598,8 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
         const int wy0 = wby + B - 2 - gr0, wx0 = wbx + B - 2 - gc0;
         const bool fast = staged && inside;
         // sweeps: 0 about the level of the iteration before; where that level or
-        // rho costs digits, 1 the target's mean (about 0), 2 its spread about the
+        // rho costs digits, or the Hessian is so near singular that the
+        // elimination inverted it, 1 the target's mean (about 0), 2 its spread about the
         // mean, 3 (ICGN) the sums with both
         for (int sweep = 0;; sweep++) {
         double sb = 0.0, sbb = 0.0, sab = 0.0, see = 0.0;
@@ -852,7 +854,7 @@ __device__ void run64_subset(const RunArgs &R, int idx, const gpv_subset_desc &d
                 gmt = tb / dn;
                 double dg2 = tbb - tb * gmt;
                 if (sweep == 0) {
-                    again = !(dg2 > kLevelDigits * tbb && rho * rho * dg2 <= kScaleDigits * saa);
+                    again = !(dg2 > kLevelDigits * tbb && rho * rho * dg2 <= kScaleDigits * saa) || !sm.flag[3];
                 } else {
                     again = sweep < 3;
                     if (sweep > 1) {  // about the mean itself
