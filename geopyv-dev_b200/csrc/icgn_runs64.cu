@@ -232,7 +232,8 @@ __device__ __noinline__ void sums_about_mean(const double2 *RG, const double *RF
 #pragma unroll 1
         for (int j = 0; j < kK; j++) {
             if (!((vm >> j) & 1)) continue;
-            const double a = RF[j * T + t] - m;
+            const double f = RF[j * T + t], a = f - m;
+            if (f != f) continue;  // a subset of NaN alone has f_m NaN and delta_f 0
             s[0] += a;
             s[1] = fma(a, a, s[1]);
             if constexpr (!FAGN) {

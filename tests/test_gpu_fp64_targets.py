@@ -192,3 +192,24 @@ def test_fagn_on_a_saturated_target_is_not_singular(oracle, gpv_mod, area, keep)
     G = gpv_mod.Image(image_gs=g, border=BORDER, keep_f64=keep)
     got = gpv_mod.solve_batch(F, G, d, precision=gpv_mod.PREC_FP64 if keep else gpv_mod.PREC_MIXED, **kw)
     assert (got["status"] == 0).mean() >= 0.95  # (a sum of roundings may still be 0: one in 200 with the kernel before the run layout)
+
+
+@pytest.mark.parametrize("method", ["icgn", "fagn"])
+def test_reference_statistics_next_to_a_pixel_that_is_nan(gpv_mod, method):
+    """A NaN pixel in f reaches 44 samples: subsets inside that square and across
+    its edge are featureless with f_m NaN, delta_f 0 where no pixel is a number
+    and NaN where some are; 45 samples away they are as without it."""
+    f = speckle()
+    clean = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    f = f.copy()
+    f[150, 150] = np.nan
+    F = gpv_mod.Image(image_gs=f, border=BORDER, keep_f64=True)
+    G = gpv_mod.Image(image_gs=np.roll(speckle(), (2, 1), (0, 1)), border=BORDER, keep_f64=True)
+    # a sample reads coefficients from 2 before to 3 after it
+    d = gpv_mod.make_desc([[150, 150], [150 + 44, 150], [150, 150 - 45 - 13], [150 + 45 + 12, 150]], 10, 1,
+                          [[1.1, 1.9] + [0.0] * 10] * 4)
+    kw = dict(precision=gpv_mod.PREC_FP64, method=method)
+    got, ref = gpv_mod.solve_batch(F, G, d, **kw), gpv_mod.solve_batch(clean, G, d, **kw)
+    assert list(got["status"]) == [2, 2, 0, 0] and np.all(np.isnan(got["f_m"][:2]))
+    assert got["delta_f"][0] == 0.0 and np.isnan(got["delta_f"][1])
+    assert np.abs(got["p"][2:] - ref["p"][2:]).max() < 1e-9 and np.abs(got["delta_f"][2:] / ref["delta_f"][2:] - 1).max() < 1e-12
