@@ -727,15 +727,17 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
             if (rigid_on) {
                 // Template pass: G(E(p)) per pixel (grain_template,
                 // src/texture.rs:213-244), zero outside the template, and the
-                // sums of G, G^2, (f - f_m) G and SDI_j G.  The template's mean,
-                // spread and gradient are the setup's fixed FP64 sums plus
-                // these, which scale with the strain, so their FP32 rounding
-                // vanishes with it.
+                // sums of G, t^2 and SDI_j G (t = f - f_m + G).  The template's
+                // mean and gradient are the setup's fixed FP64 sums plus these,
+                // which scale with the strain, so their FP32 rounding vanishes
+                // with it.  Its spread is its own sum: as a difference of sums of
+                // f^2, f G and G^2 a strain that cancels f (its trace 1, where
+                // the pixels have no grain) left their rounding, or 0.
                 const float s2f = (float)A.grain_scal[2], fmsf = (float)((double)shift - fm);
                 const float2 px2 = make_float2(ORDER == 2 ? (float)sm.p[6 % M] : 0.f, ORDER == 2 ? (float)sm.p[7 % M] : 0.f);
                 const float2 pxy = make_float2(ORDER == 2 ? (float)sm.p[8 % M] : 0.f, ORDER == 2 ? (float)sm.p[9 % M] : 0.f);
                 const float2 py2 = make_float2(ORDER == 2 ? (float)sm.p[10 % M] : 0.f, ORDER == 2 ? (float)sm.p[11 % M] : 0.f);
-                double g1 = 0.0, g2 = 0.0, gf = 0.0;
+                double g1 = 0.0, t2 = 0.0;
                 KSum unused[3];
                 float2 TB[6];
 #pragma unroll
@@ -748,6 +750,7 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                     RunAcc ac;
                     ac.p1 = ac.p2 = ac.pfg = 0.f;
                     ac.m0 = ac.m1 = ac.m2 = make_float2(0.f, 0.f);
+                    float tt = 0.f;
                     // the run's records and grain samples together in flight (the
                     // stores of G below would order the loads after them)
                     float4 rcs[K];
@@ -777,17 +780,18 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                         rc.z += fmsf;  // f - f_m
                         const float G = (-0.5f * s2f * (e0 * h0 + e1 * h1 + 2.0f * e2 * h2) - (e0 + e1) * rc.z) * rc.w;
                         RTG[sl] = G;
+                        const float tm = fmaf(rc.z, rc.w, G);
+                        tt = fmaf(tm, tm, tt);
                         acc_sample<ORDER, false>(ac, unused, rc, G, 0.f, make_float2(dyf, dyf), make_float2(dyf * dyf, dyf * dyf));
                     }
                     g1 += (double)ac.p1;
-                    g2 += (double)ac.p2;
-                    gf += (double)ac.pfg;
+                    t2 += (double)tt;
                     acc_expand<ORDER>(ac, dxf, TB);
                 }
                 double *dst = sm.red2[wid];
-                const double gv[3] = {g1, g2, gf};
+                const double gv[2] = {g1, t2};
 #pragma unroll
-                for (int q = 0; q < 3; q++) {
+                for (int q = 0; q < 2; q++) {
                     const double t = warp_sum(gv[q]);
                     if (lane == q) dst[q] = t;
                 }
@@ -968,11 +972,11 @@ __device__ void run_subset(const RunArgs &R, int idx, const gpv_subset_desc &d, 
                         for (int w = 0; w < NT / 32; w++) tq += sm.red2[w][lane];
                     }
                     const double q0 = __shfl_sync(0xffffffffu, tq, 0), q1 = __shfl_sync(0xffffffffu, tq, 1);
-                    const double q2 = __shfl_sync(0xffffffffu, tq, 2);
                     sgj = __shfl_down_sync(0xffffffffu, tq, 3);  // lane j: sum SDI_j G
                     tmf = q0 * inv_dn;
-                    dref = sqrt(fmax(saa + 2.0 * q2 + q1 - q0 * tmf, 0.0));
-                    inv_dref = 1.0 / dref;
+                    const double dt2 = q1 - q0 * tmf;
+                    dref = sqrt(dt2 < 0.0 ? 0.0 : dt2);
+                    inv_dref = dref > 0.0 ? 1.0 / dref : __longlong_as_double(0x7ff8000000000000ll);  // no template, no ZNCC
                     sab -= tmf * t0;
                 }
             }

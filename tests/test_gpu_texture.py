@@ -222,3 +222,30 @@ def test_rigid_residual_map_and_record(gpv_mod):
     assert rms[1] < 0.5 * rms[0]
     # the subset's reference values are the image's spline at its pixels
     assert np.abs(sub.f - F.eval(sub.f_coords)).max() == 0.0
+
+
+@pytest.mark.parametrize("trace", [1.0003, 0.9993, 0.9, 1.3])
+@pytest.mark.parametrize("order", [1, 2])
+def test_a_template_that_its_strain_cancels_has_its_own_spread(gpv_mod, oracle, order, trace):
+    """Where the pixels carry no grain (a black area whose edge rings in the
+    coefficients) the template is (1 - tr E)(f - f_m): at tr E = 1.0003 it keeps 1e-7 of
+    f's second moment, below the rounding of FP32 sums of its parts (a spread of 0,
+    a ZNCC of infinity, a subset of good quality).  Its ZNCC against an unrelated
+    target is the oracle's: FP32 grey levels leave 6e-8 / 3e-4 of the template, so 0.01."""
+    from test_gpu_fp64_targets import speckle
+    f, g = speckle(7), speckle(8)
+    f[150:] = 0.0
+    r = np.random.default_rng(3)
+    n = 40
+    d = np.zeros((n, 12))
+    d[:, 0] = 0.3
+    d[:, 2] = d[:, 5] = np.sqrt(1.0 + trace) - 1.0
+    d = gpv_mod.make_desc(np.stack([r.uniform(40, 260, n), r.uniform(272, 277, n)], 1), 25, order, d)
+    kw = dict(max_iterations=1)
+    ref = oracle.solve_batch(oracle.get_c(f, 3), oracle.get_c(g, 3), f.shape, 3, d, grain=oracle.grain(f), **kw)
+    ok = (ref["status"] == 0) & (ref["delta_f"] > 0.1)
+    assert ok.sum() >= 20
+    F, G = gpv_mod.Image(image_gs=f, border=3), gpv_mod.Image(image_gs=g, border=3)
+    got = gpv_mod.solve_batch(F, G, d, texture="rigid", **kw)
+    assert not got["quality_ok"].any() and np.all(got["texture"][ok] == 1)
+    assert np.abs(got["c_zncc"] - ref["c_zncc"])[ok].max() < 0.01
