@@ -213,3 +213,22 @@ def test_reference_statistics_next_to_a_pixel_that_is_nan(gpv_mod, method):
     assert list(got["status"]) == [2, 2, 0, 0] and np.all(np.isnan(got["f_m"][:2]))
     assert got["delta_f"][0] == 0.0 and np.isnan(got["delta_f"][1])
     assert np.abs(got["p"][2:] - ref["p"][2:]).max() < 1e-9 and np.abs(got["delta_f"][2:] / ref["delta_f"][2:] - 1).max() < 1e-12
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_a_mesh_over_a_saturated_half_is_solved(gpv_mod, order):
+    """FAGN on FP32 coefficients: nodes on the saturated half are not called
+    singular, which would end the mesh, nor matched; the others are solved."""
+    f = speckle(3, 400).round().clip(0, 255)
+    g = np.roll(f, (1, 2), (0, 1))
+    g[:, 230:] = 255.0
+    X, Y = np.meshgrid(np.linspace(50, 350, 9), np.linspace(50, 350, 9))
+    nodes = np.stack([X.ravel(), Y.ravel()], 1)
+    i = np.arange(81).reshape(9, 9)
+    a, b, c, e = i[:-1, :-1].ravel(), i[:-1, 1:].ravel(), i[1:, :-1].ravel(), i[1:, 1:].ravel()
+    elements = np.concatenate([np.stack([a, b, c], 1), np.stack([b, e, c], 1)])
+    m = gpv_mod.Mesh(nodes, elements, gpv_mod.Image(image_gs=f), gpv_mod.Image(image_gs=g))
+    m.solve(20, [87.5, 87.5], [2.0, 1.0] + [0.0] * (6 * order - 2), subset_order=order, method="fagn",
+            preconditioning="layer-RG", override_active=True)
+    assert m.quality_ok[nodes[:, 0] < 200].all() and not m.quality_ok[nodes[:, 0] > 260].any()
+    assert np.all(m.c_zncc[nodes[:, 0] > 260] < 0.75)
